@@ -14,6 +14,7 @@ DDIM and PLMS, guided and unguided, latents of 32x32 and 64x64.
 import math
 
 import torch
+import torch.nn.functional as F
 
 import modiff_b200 as m
 from modiff_b200.ldm_unet import LSUN_CHURCHES_KL8, SD_V1
@@ -232,3 +233,46 @@ def tolerance(case):
             return {"rel": 0.03, "max": 0.3}
         return {"rel": 0.0012, "max": 0.006} if case["static"] else {"rel": 0.006, "max": 0.025}
     return {"rel": 0.002, "max": 0.008} if kind == "ldm" else {"rel": 0.013, "max": 0.05}
+
+
+def _conv64(x, p, name):
+    """Stride-1 'same' convolution in 64 bits, one image at a time as a matrix product."""
+    w, b = p[name + ".weight"], p[name + ".bias"]
+    k = w.shape[-1]
+    images = [(w.flatten(1) @ F.unfold(im[None], k, padding=k // 2)[0]).view(-1, *x.shape[2:])
+              for im in x]
+    return torch.stack(images) + b.view(1, -1, 1, 1)
+
+
+def _norm64(x, p, name, silu=True):
+    y = F.group_norm(x, 32, p[name + ".weight"], p[name + ".bias"], eps=1e-6)
+    return F.silu(y) if silu else y
+
+
+def _block64(x, p, name):
+    h = _conv64(_norm64(x, p, name + ".norm1"), p, name + ".conv1")
+    h = _conv64(_norm64(h, p, name + ".norm2"), p, name + ".conv2")
+    return h + (_conv64(x, p, name + ".nin_shortcut") if name + ".nin_shortcut.weight" in p else x)
+
+
+def exact(case, seed):
+    """The decoder in plain 64-bit torch.  A sampler has no such value: it rounds residuals of
+    nearly equal tensors to codes, and where a code falls decides more than any sum's precision."""
+    if not case["net"].startswith("decoder"):
+        return None
+    state = prepare(case, seed)
+    p = {k.removeprefix("decoder."): v.double() for k, v in state["decoder"].state_dict().items()}
+    h = _conv64(_conv64(state["z"].double(), p, "post_quant_conv"), p, "conv_in")
+    h = _block64(h, p, "mid.block_1")
+    n = _norm64(h, p, "mid.attn_1.norm", silu=False)
+    q, k, v = (_conv64(n, p, "mid.attn_1." + s).flatten(2) for s in "qkv")
+    a = torch.softmax(q.transpose(1, 2) @ k * q.shape[1] ** -0.5, dim=2) @ v.transpose(1, 2)
+    h = h + _conv64(a.transpose(1, 2).reshape(h.shape), p, "mid.attn_1.proj_out")
+    h = _block64(h, p, "mid.block_2")
+    for level in (3, 2, 1, 0):
+        for i in range(3):
+            h = _block64(h, p, f"up.{level}.block.{i}")
+        if level:
+            h = _conv64(F.interpolate(h, scale_factor=2.0, mode="nearest"), p,
+                        f"up.{level}.upsample.conv")
+    return _conv64(_norm64(h, p, "norm_out"), p, "conv_out")
