@@ -399,6 +399,26 @@ int modiff_im2col_codes(const int8_t* codes, int8_t* out, const modiff_conv_geom
 int modiff_conv_fp32(const float* x, const float* w_kn, const float* bias, float* out,
                      const modiff_conv_geom* g, void* stream);
 
+/* The same convolution (stride 1, no split; qdiff/quant_layer.py:309-311) at fp32 precision on the
+ * tensor cores: each fp32 operand as three bf16 planes that sum to it exactly.
+ *   modiff_f32_split_weights  w fp32 [cout][cin][kh][kw] -> weight planes (modiff_f32_weights_bytes)
+ *   modiff_f32_split          x fp32 NCHW -> activation planes (modiff_f32_planes_bytes); on the way
+ *       GroupNorm (groups > 0: gamma, beta, eps and modiff_f32_norm_bytes of work), SiLU, and, with
+ *       up2, nearest x2 upsampling: x is then [batch][cin][h/2][w/2] for a geometry of h x w
+ *       (ldm/modules/diffusionmodules/model.py:45-60, 114-134)
+ *   modiff_conv_f32_tc        out = conv + bias, or residual + (conv + bias); bias / residual may be
+ *       NULL.  Sums of infinities and NaN are those of modiff_conv_fp32.
+ * Planes are 16-byte aligned. */
+int64_t modiff_f32_planes_bytes(const modiff_conv_geom* g);
+int64_t modiff_f32_weights_bytes(const modiff_conv_geom* g);
+int64_t modiff_f32_norm_bytes(const modiff_conv_geom* g, int groups);
+int modiff_f32_split_weights(const float* w, uint16_t* out, const modiff_conv_geom* g, void* stream);
+int modiff_f32_split(const float* x, const modiff_conv_geom* g, int up2, const float* gamma,
+                     const float* beta, int groups, float eps, int silu, void* work, uint16_t* planes,
+                     void* stream);
+int modiff_conv_f32_tc(const uint16_t* planes, const uint16_t* wplanes, const float* bias,
+                       const float* residual, float* out, const modiff_conv_geom* g, void* stream);
+
 /* ---- split-bf16 tensor-core GEMM (first sampling step and attention matmuls) -------------
  * fp32 values travel as two bf16 planes, hi = bf16(x) and lo = bf16(x - hi); the GEMM adds the
  * products hi*hi + hi*lo + lo*hi in fp32 (relative error ~1e-5). */

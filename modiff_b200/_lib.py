@@ -104,6 +104,12 @@ SIGNATURES = {
                                         _P]),
     "modiff_im2col_codes": (C.c_int, [_P, _P, _G, C.c_int, _P]),
     "modiff_conv_fp32": (C.c_int, [_P, _P, _P, _P, _G, _P]),
+    "modiff_f32_planes_bytes": (C.c_int64, [_G]),
+    "modiff_f32_weights_bytes": (C.c_int64, [_G]),
+    "modiff_f32_norm_bytes": (C.c_int64, [_G, C.c_int]),
+    "modiff_f32_split_weights": (C.c_int, [_P, _P, _G, _P]),
+    "modiff_f32_split": (C.c_int, [_P, _G, C.c_int, _P, _P, C.c_int, C.c_float, C.c_int, _P, _P, _P]),
+    "modiff_conv_f32_tc": (C.c_int, [_P, _P, _P, _P, _P, _G, _P]),
     "modiff_bf16_planes_bytes": (C.c_int64, [_G]),
     "modiff_split_bf16": (C.c_int, [_P, _P, _G, _P]),
     "modiff_split_bf16_rows": (C.c_int, [_P, _P, C.c_int64, C.c_int, C.c_int, C.c_int, C.c_int, _P]),
@@ -174,6 +180,7 @@ KERNELS_PER_CALL = {
     "modiff_quantize_static": 1, "modiff_i8_mma_probe": 1, "modiff_wait_probe": 1,
     "modiff_attn_quantize": 2, "modiff_attention_i8": 1, "modiff_adaround_fake_quant": 1,
     "modiff_pack_weights_int4": 1, "modiff_igemm_conv_packed4": 1,
+    "modiff_f32_split_weights": 1, "modiff_f32_split": 1, "modiff_conv_f32_tc": 1,
 }
 LAUNCHES = [0]        # kernels launched through `call` since import
 # Bumped whenever a layer allocates or replaces a device buffer that kernels address directly

@@ -22,9 +22,10 @@ def _normalize(channels):
     return nn.GroupNorm(num_groups=32, num_channels=channels, eps=1e-6, affine=True)
 
 
-def _run_conv(conv, x):
-    """An fp32 convolution on the library's kernel: the layer is wrapped once in a QuantModule
-    left in its unquantised state (qdiff/quant_layer.py:309-311, the plain-convolution branch)."""
+def _run_conv(conv, x, **around):
+    """A plain convolution on the library's kernels, `around` being what is evaluated with it
+    (QuantModule.conv_plain): the layer is wrapped once in a QuantModule left in its unquantised
+    state (qdiff/quant_layer.py:309-311, the plain-convolution branch)."""
     key = (conv.weight.data_ptr(), conv.weight._version,
            None if conv.bias is None else conv.bias._version)
     runner = conv.__dict__.get("_modiff_runner")
@@ -35,7 +36,7 @@ def _run_conv(conv, x):
                               'scale_method': 'max', 'leaf_param': True, 'dynamic': True})
         conv.__dict__["_modiff_runner"] = runner      # not a submodule: state_dict keys stay
         conv.__dict__["_modiff_runner_key"] = key
-    return runner(x)
+    return runner.conv_plain(x, **around)
 
 
 class ResnetBlock(nn.Module):
@@ -61,11 +62,10 @@ class ResnetBlock(nn.Module):
                 self.nin_shortcut = nn.Conv2d(in_channels, out_channels, 1, 1, 0)
 
     def forward(self, x, temb=None):
-        h = _run_conv(self.conv1, ops.groupnorm(x, self.norm1, True))
-        h = _run_conv(self.conv2, ops.groupnorm(h, self.norm2, True))
+        h = _run_conv(self.conv1, x, norm=self.norm1, silu=True)
         if self.in_channels != self.out_channels:
             x = _run_conv(self.conv_shortcut if self.use_conv_shortcut else self.nin_shortcut, x)
-        return ops.add(x, h)
+        return _run_conv(self.conv2, h, norm=self.norm2, silu=True, residual=x)
 
 
 class AttnBlock(nn.Module):
@@ -86,7 +86,7 @@ class AttnBlock(nn.Module):
         b, c, h, w = q.shape
         a = ops.attention(q.reshape(b, c, h * w), k.reshape(b, c, h * w),
                               v.reshape(b, c, h * w), float(int(c) ** (-0.5)))
-        return ops.add(x, _run_conv(self.proj_out, a.reshape(b, c, h, w)))
+        return _run_conv(self.proj_out, a.reshape(b, c, h, w), residual=x)
 
 
 class Upsample(nn.Module):
@@ -99,8 +99,7 @@ class Upsample(nn.Module):
             self.conv = nn.Conv2d(in_channels, in_channels, 3, 1, 1)
 
     def forward(self, x):
-        x = ops.upsample2x(x)
-        return _run_conv(self.conv, x) if self.with_conv else x
+        return _run_conv(self.conv, x, up2=True) if self.with_conv else ops.upsample2x(x)
 
 
 class Decoder(nn.Module):
@@ -170,7 +169,7 @@ class Decoder(nn.Module):
                 h = level.upsample(h)
         if self.give_pre_end:
             return h
-        h = _run_conv(self.conv_out, ops.groupnorm(h, self.norm_out, True))
+        h = _run_conv(self.conv_out, h, norm=self.norm_out, silu=True)
         return torch.tanh(h) if self.tanh_out else h
 
 

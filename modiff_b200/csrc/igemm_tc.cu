@@ -823,6 +823,7 @@ int read_device_status_modq(int* status, int reset);        // modq.cu
 int read_device_status_probe(int* status, int reset);       // i8_probe.cu
 int read_device_status_pair(int* status, int reset);        // igemm_pair.cu
 int read_device_status_attention_i8(int* status, int reset);   // attention_i8.cu
+int read_device_status_conv_f32(int* status, int reset);       // conv_f32_tc.cu
 bool pair_supported(const modiff_conv_geom* g, int with_sum_rows, int per_sample, const float* bias,
                     const int32_t* acc_out, const float* o_hat);
 int launch_igemm_pair(const int8_t* codes, const int8_t* wcodes, int with_sum_rows,
@@ -875,7 +876,10 @@ int read_device_status(int* status, int reset) {
   int i8 = 0;
   rc = read_device_status_attention_i8(&i8, reset);
   if (rc) return rc;
-  *status = a | b | c | d | e | f | h | i8;
+  int f32 = 0;
+  rc = read_device_status_conv_f32(&f32, reset);
+  if (rc) return rc;
+  *status = a | b | c | d | e | f | h | i8 | f32;
   return MODIFF_OK;
 }
 

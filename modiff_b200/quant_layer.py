@@ -219,6 +219,7 @@ class QuantModule(nn.Module):
         self._geom_buffers = {}
         self._wpack = None
         self._org_kn = None
+        self._org_planes = None
         self._loaded_act_scale = None   # (delta per segment, zero point per segment) to install
         self._a_hat_half = False        # a_hat held at the input resolution of an Upsample block
         self.implicit_pad = (0, 0, 0, 0)   # extra (left, right, top, bottom) zero padding
@@ -420,12 +421,28 @@ class QuantModule(nn.Module):
         self._wpack = pack
         return pack
 
-    def _org_weights_kn(self):
-        """Unquantised weights as [cin*kh*kw][cout] for the fp32 kernel."""
+    def _org_weights_planes(self, g):
+        """Unquantised weights as the three bf16 planes of modiff_conv_f32_tc."""
+        self._org_to_device()
+        w = self.org_weight
+        key = (w.data_ptr(), w._version)
+        if self._org_planes is None or self._org_planes[0] != key:
+            planes = torch.empty(_lib.lib().modiff_f32_weights_bytes(C.byref(g)) // 2,
+                                 dtype=torch.int16, device=w.device)
+            _lib.call('modiff_f32_split_weights', w.contiguous().data_ptr(), planes.data_ptr(),
+                      C.byref(g), _lib.stream_ptr())
+            self._org_planes = (key, planes)
+        return self._org_planes[1]
+
+    def _org_to_device(self):
         if self.org_weight.device != self.weight.device:   # plain attribute: .to() skips it
             self.org_weight = self.org_weight.to(self.weight.device)
             if self.org_bias is not None:
                 self.org_bias = self.org_bias.to(self.weight.device)
+
+    def _org_weights_kn(self):
+        """Unquantised weights as [cin*kh*kw][cout] for the fp32 kernel."""
+        self._org_to_device()
         w = self.org_weight
         key = (w.data_ptr(), w._version)
         if self._org_kn is None or self._org_kn[0] != key:
@@ -445,6 +462,57 @@ class QuantModule(nn.Module):
         _lib.call('modiff_conv_fp32', x.data_ptr(), w_kn.data_ptr(), _lib.ptr(bias),
                   out.data_ptr(), C.byref(g), _lib.stream_ptr(),
                   nbytes=4 * (x.numel() + out.numel() + w_kn.numel()))
+
+    def conv_plain(self, x, norm=None, silu=False, up2=False, residual=None):
+        """The unquantised layer (quant_layer.py:309-311) on x, or on what GroupNorm (`norm`), SiLU
+        and nearest x2 upsampling (`up2`) make of it, plus `residual`.  Stride-1 convolutions from
+        32 input channels on run on the tensor cores, which evaluate all of that around the
+        convolution (modiff_conv_f32_tc); with fewer the padding of K to 64 channels per tap
+        would outweigh the faster products, and the fp32 kernel takes the layer."""
+        from . import ops
+        _lib.require_cuda(x, "QuantModule input")
+        x = x.contiguous()
+        shape = tuple(x.shape)
+        if up2:
+            shape = shape[:2] + (2 * shape[2], 2 * shape[3])
+        g = self._geom(torch.empty(shape, device='meta'), 0)
+        ho_wo = _lib.out_hw(g)
+        out = torch.empty(self._shape_from(x, g, ho_wo), dtype=torch.float32, device=x.device)
+        if residual is not None:
+            _lib.require_cuda(residual, "residual")
+            residual = residual.contiguous()
+            if tuple(residual.shape) != tuple(out.shape):
+                raise ModiffError(f"residual {tuple(residual.shape)} does not match the output "
+                                  f"{tuple(out.shape)}")
+        if norm is not None and norm.num_channels != g.cin:
+            raise ModiffError(f"GroupNorm expects {norm.num_channels} channels, got {g.cin}")
+        if g.stride != 1 or g.cin < 32 or self.fwd_func is F.linear:
+            if norm is not None:
+                x = ops.groupnorm(x, norm, silu)
+            elif silu:
+                x = ops.silu(x)
+            if up2:
+                x = ops.upsample2x(x)
+            self._conv_fp32(x, self._org_weights_kn(), self.org_bias, g, out)
+            return out if residual is None else ops.add(residual, out)
+        l = _lib.lib()
+        dev = x.device
+        groups = 0 if norm is None else norm.num_groups
+        planes = torch.empty(l.modiff_f32_planes_bytes(C.byref(g)) // 2, dtype=torch.int16, device=dev)
+        work = torch.empty(l.modiff_f32_norm_bytes(C.byref(g), groups), dtype=torch.uint8, device=dev) \
+            if groups else None
+        weights = self._org_weights_planes(g)
+        _lib.call('modiff_f32_split', x.data_ptr(), C.byref(g), int(up2),
+                  None if norm is None else norm.weight.data_ptr(),
+                  None if norm is None else norm.bias.data_ptr(), groups,
+                  0.0 if norm is None else float(norm.eps), int(silu), _lib.ptr(work),
+                  planes.data_ptr(), _lib.stream_ptr())
+        if groups:
+            _lib.LAUNCHES[0] += 2              # the statistics: pieces, slabs
+        _lib.call('modiff_conv_f32_tc', planes.data_ptr(), weights.data_ptr(),
+                  _lib.ptr(self.org_bias), _lib.ptr(residual), out.data_ptr(), C.byref(g),
+                  _lib.stream_ptr(), nbytes=4 * (x.numel() + out.numel() + self.weight.numel()))
+        return out
 
     @staticmethod
     def _bf16_ok(g, ho_wo):
@@ -862,12 +930,7 @@ class QuantModule(nn.Module):
             input = input.contiguous()
 
         if not self.use_weight_quant and not self.use_act_quant and not self.modulate:
-            g = self._geom(input, 0)
-            buf_ho_wo = _lib.out_hw(g)
-            out = torch.empty(self._shape_from(input, g, buf_ho_wo), dtype=torch.float32,
-                              device=input.device)
-            self._conv_fp32(input, self._org_weights_kn(), self.org_bias, g, out)
-            return self.activation_function(out)
+            return self.activation_function(self.conv_plain(input))
 
         if split != 0:
             if self.split != 0:

@@ -1,0 +1,79 @@
+"""The tensor-core fp32 convolution (three bf16 planes per operand) against the same convolution in
+64 bits, at the edges of its tiles: ragged channel counts, one chunk and several, widths that are
+not powers of two, images smaller than a tile, few output channels."""
+import pytest
+import torch
+import torch.nn.functional as F
+
+pytestmark = pytest.mark.gpu
+
+
+def _layer(conv):
+    import modiff_b200 as m
+    return m.QuantModule(conv, {'n_bits': 8, 'channel_wise': True, 'scale_method': 'max'},
+                         {'n_bits': 8, 'symmetric': True, 'channel_wise': False,
+                          'scale_method': 'max', 'leaf_param': True, 'dynamic': True})
+
+
+def _bound(x, w, pad):
+    """Products are exact to 2^-25; a chunk of 64 channels adds 24 terms in the tensor core, each
+    rounded (or cut off) at 2^-23 of a partial sum that stays below sum |x||w|, and the chunks and
+    the bias are added in fp32."""
+    chunks = w.shape[2] * w.shape[3] * -(-w.shape[1] // 64)
+    return (24 + chunks + 2) * 2.0 ** -23 * F.conv2d(x.abs(), w.abs(), padding=pad) + 1e-30
+
+
+@pytest.mark.parametrize("b,cin,cout,h,w,k,pad", [
+    (1, 32, 16, 8, 8, 3, 1), (3, 40, 3, 5, 7, 3, 1), (1, 64, 128, 16, 16, 1, 0),
+    (2, 130, 72, 24, 24, 3, 1), (1, 128, 3, 4, 512, 3, 1), (130, 64, 20, 1, 1, 1, 0),
+    (5, 96, 200, 6, 40, 5, 2), (1, 512, 512, 32, 32, 3, 1), (1, 256, 130, 64, 128, 3, 0)])
+def test_matches_64_bit_convolution(cuda, b, cin, cout, h, w, k, pad):
+    import modiff_b200 as m
+    torch.manual_seed(b + cin)
+    conv = torch.nn.Conv2d(cin, cout, k, padding=pad).to(cuda)
+    x = torch.randn(b, cin, h, w, device=cuda) * torch.rand(b, cin, 1, 1, device=cuda) * 3
+    y = _layer(conv)(x)
+    torch.cuda.synchronize()
+    assert m.device_status() == 0
+    wd, bd = conv.weight.detach().double().cpu(), conv.bias.detach().double().cpu()
+    xd = x.double().cpu()
+    ref = F.conv2d(xd, wd, bd, padding=pad)
+    err = (y.double().cpu() - ref).abs()
+    bound = _bound(xd, wd, pad) + 2.0 ** -23 * ref.abs()
+    assert bool((err <= bound).all()), float((err / bound).max())
+
+
+@pytest.mark.parametrize("b,cin,cout,h,w,up2", [(2, 64, 32, 8, 8, False), (1, 96, 40, 7, 5, False),
+                                                (1, 128, 128, 64, 96, False), (2, 64, 48, 5, 6, True)])
+def test_norm_silu_upsample_and_residual_around_the_convolution(cuda, b, cin, cout, h, w, up2):
+    torch.manual_seed(7)
+    conv = torch.nn.Conv2d(cin, cout, 3, padding=1).to(cuda)
+    norm = torch.nn.GroupNorm(32, cin, eps=1e-6).to(cuda)
+    with torch.no_grad():
+        norm.weight.normal_(1.0, 0.3)
+        norm.bias.normal_()
+    x = torch.randn(b, cin, h, w, device=cuda) + 4.0
+    s = 2 if up2 else 1
+    res = torch.randn(b, cout, s * h, s * w, device=cuda)
+    y = _layer(conv).conv_plain(x, norm=norm, silu=True, up2=up2, residual=res)
+    n = F.silu(F.group_norm(x.double(), 32, norm.weight.double(), norm.bias.double(), 1e-6))
+    if up2:
+        n = F.interpolate(n, scale_factor=2.0, mode="nearest")
+    ref = F.conv2d(n.cpu(), conv.weight.double().cpu(), conv.bias.double().cpu(), padding=1) + res.double().cpu()
+    # fp32 GroupNorm of values around 4 (mean subtracted: 2^-22 of 4 over a deviation of 1) and a
+    # SiLU of about 2 ulp, both multiplied through the sum of |w|: 1e-5 of the largest value
+    assert float((y.double().cpu() - ref).abs().max() / ref.abs().max()) < 1e-5
+
+
+def test_infinities_and_large_values_are_those_of_the_plain_sum(cuda):
+    torch.manual_seed(9)
+    conv = torch.nn.Conv2d(64, 16, 3, padding=1).to(cuda)
+    x = torch.randn(1, 64, 8, 8, device=cuda)
+    x[0, 3, 1, 1], x[0, 5, 6, 6], x[0, 9, 1, 6] = float("inf"), float("nan"), 3.4e38
+    y = _layer(conv)(x).cpu()
+    ref = F.conv2d(x.cpu(), conv.weight.detach().cpu(), conv.bias.detach().cpu(), padding=1)
+    assert torch.equal(torch.isnan(y), torch.isnan(ref))
+    assert torch.equal(torch.isinf(y), torch.isinf(ref))
+    assert torch.equal(y[torch.isinf(y)], ref[torch.isinf(ref)])
+    fin = torch.isfinite(ref)
+    assert torch.allclose(y[fin], ref[fin], rtol=1e-5, atol=1e-4)
