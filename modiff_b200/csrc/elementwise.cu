@@ -117,38 +117,64 @@ groupnorm_silu_kernel(const float* __restrict__ x0, const float* __restrict__ x1
   }
 }
 
-// Attention for small token counts (t, tk <= 64): one block per image, fp32 on CUDA cores.
+// Attention for small token counts (t, tk <= 64), fp32 on CUDA cores:
 // q [c][t], k [c][tk], v [c][tk], out [c][t]  (qdiff/quant_block.py:344-360).
-__global__ void __launch_bounds__(256)
+// A block owns 8 queries of an image; what bounds it is the chain of loads along the channels, so
+// the threads that the score pairs leave over split the channels (each slice's loads are
+// independent and issued four at a time) and the slices are added at the end.  (One block of 256
+// threads per image, each walking all channels of its pairs, took 46 us for one image of 16 tokens
+// and 256 channels.)
+constexpr int kSmallQ = 8, kSmallThreads = 512;
+__global__ void __launch_bounds__(kSmallThreads)
 attention_small_kernel(const float* __restrict__ q, const float* __restrict__ k,
                        const float* __restrict__ v, float* __restrict__ out, int c, int t, int tk,
-                       float scale) {
-  __shared__ float sc[64][65];
+                       int lg_pairs, float scale) {
+  __shared__ float part[kSmallThreads];
+  __shared__ float sc[kSmallQ][65];
   const int b = blockIdx.x;
-  const float* qb = q + (size_t)b * c * t;
+  const int i0 = blockIdx.y * kSmallQ;
+  const int nq = min(kSmallQ, t - i0);
+  const float* qb = q + (size_t)b * c * t + i0;
   const float* kb = k + (size_t)b * c * tk;
   const float* vb = v + (size_t)b * c * tk;
-  for (int e = threadIdx.x; e < t * tk; e += blockDim.x) {
-    const int i = e / tk, j = e % tk;
-    float acc = 0.0f;
-    for (int ch = 0; ch < c; ++ch) acc = fmaf(__ldg(qb + (size_t)ch * t + i), __ldg(kb + (size_t)ch * tk + j), acc);
-    sc[i][j] = acc * scale;
+  const int pairs = nq * tk;                         // <= 1 << lg_pairs <= kSmallThreads
+  const int slices = kSmallThreads >> lg_pairs;
+  const int e = threadIdx.x & ((1 << lg_pairs) - 1), slice = threadIdx.x >> lg_pairs;
+  float acc = 0.0f;
+  if (e < pairs) {
+    const float* qi = qb + e / tk;
+    const float* kj = kb + e % tk;
+#pragma unroll 4
+    for (int ch = slice; ch < c; ch += slices)
+      acc = fmaf(__ldg(qi + (size_t)ch * t), __ldg(kj + (size_t)ch * tk), acc);
+  }
+  part[threadIdx.x] = acc;
+  __syncthreads();
+  if (threadIdx.x < pairs) {
+    for (int s = 1; s < slices; ++s) acc += part[(s << lg_pairs) + e];
+    sc[e / tk][e % tk] = acc * scale;
   }
   __syncthreads();
-  for (int i = threadIdx.x; i < t; i += blockDim.x) {
-    float mx = -INFINITY;
-    for (int j = 0; j < tk; ++j) mx = fmaxf(mx, sc[i][j]);
-    float sum = 0.0f;
-    for (int j = 0; j < tk; ++j) { const float e = expf(sc[i][j] - mx); sc[i][j] = e; sum += e; }
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  if (warp < nq) {                                   // one warp per query, two keys per lane
+    const float a0 = lane < tk ? sc[warp][lane] : -INFINITY;
+    const float a1 = lane + 32 < tk ? sc[warp][lane + 32] : -INFINITY;
+    float mx = fmaxf(a0, a1);
+    for (int o = 16; o > 0; o >>= 1) mx = fmaxf(mx, __shfl_xor_sync(0xffffffffu, mx, o));
+    const float e0 = lane < tk ? expf(a0 - mx) : 0.0f, e1 = lane + 32 < tk ? expf(a1 - mx) : 0.0f;
+    float sum = e0 + e1;
+    for (int o = 16; o > 0; o >>= 1) sum += __shfl_xor_sync(0xffffffffu, sum, o);
     const float inv = 1.0f / sum;
-    for (int j = 0; j < tk; ++j) sc[i][j] *= inv;
+    if (lane < tk) sc[warp][lane] = e0 * inv;
+    if (lane + 32 < tk) sc[warp][lane + 32] = e1 * inv;
   }
   __syncthreads();
-  for (int e = threadIdx.x; e < c * t; e += blockDim.x) {
-    const int ch = e / t, i = e % t;
-    float acc = 0.0f;
-    for (int j = 0; j < tk; ++j) acc = fmaf(__ldg(vb + (size_t)ch * tk + j), sc[i][j], acc);
-    out[(size_t)b * c * t + e] = acc;
+  for (int o = threadIdx.x; o < c * nq; o += kSmallThreads) {
+    const int ch = o / nq, i = o % nq;
+    float r = 0.0f;
+#pragma unroll 4
+    for (int j = 0; j < tk; ++j) r = fmaf(__ldg(vb + (size_t)ch * tk + j), sc[i][j], r);
+    out[((size_t)b * c + ch) * t + i0 + i] = r;
   }
 }
 
@@ -400,7 +426,10 @@ int modiff_attention_small(const float* q, const float* k, const float* v, float
                            int c, int t, int tk, float scale, void* stream) {
   MODIFF_CHECK_ARG(q && k && v && out && batch > 0 && c > 0, "bad argument");
   MODIFF_CHECK_ARG(t > 0 && tk > 0 && t <= 64 && tk <= 64, "token counts %d x %d exceed 64", t, tk);
-  attention_small_kernel<<<batch, 256, 0, (cudaStream_t)stream>>>(q, k, v, out, c, t, tk, scale);
+  int lg = 0;
+  while ((1 << lg) < (t < kSmallQ ? t : kSmallQ) * tk) ++lg;
+  attention_small_kernel<<<dim3(batch, ceil_div(t, kSmallQ)), kSmallThreads, 0, (cudaStream_t)stream>>>(
+      q, k, v, out, c, t, tk, lg, scale);
   MODIFF_LAUNCH_CHECK("attention_small_kernel");
   return MODIFF_OK;
 }

@@ -1144,6 +1144,10 @@ class QuantModule(nn.Module):
     # ------------------------------------------------------------------ grouped small linears
     group_small_linears = os.environ.get("MODIFF_LINEAR_GROUP", "1") != "0"
     _GROUP_MAX_ROWS = 512
+    # Multiply-adds per layer up to which one dp4a launch beats a tensor-core launch per layer
+    # (about 8.7 us each).  Measured, group / separate: 64 rows x 1280 -> 3 x 1280 (105 M a layer)
+    # 21 / 34 us, 128 rows (210 M) 32 / 26 us, 512 rows (839 M) 125 / 26 us.
+    _GROUP_MAX_MACS = 150e6
 
     def _group_register(self, member, g):
         """Called on the first step by a layer that shares this layer's codes.  Small linear
@@ -1165,6 +1169,9 @@ class QuantModule(nn.Module):
         if not members or self.fwd_func is not F.linear or g.split != 0:
             return False
         layers = [self] + members
+        if g.batch * g.cin * sum(m.weight.shape[0] for m in layers) > \
+                self._GROUP_MAX_MACS * len(layers):
+            return False                     # each layer on the tensor cores
         for m in members:
             if m.a_hat is not self.a_hat or m.o_hat is None or m._wpack is None:
                 return False
