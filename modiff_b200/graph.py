@@ -4,7 +4,9 @@ From the third call after a `reset_cache()` every step launches the same kernels
 buffers (the first call is the unquantised step that creates the caches, the second is the
 first quantised one and allocates the code buffers): that launch sequence - several hundred
 small kernels - is captured once per input shape and replayed, which removes the per-launch
-host cost.  The reference has no counterpart (it runs eager PyTorch, with host synchronisations
+host cost.  In later passes the buffers are there from the start, so the second call launches
+that sequence too and is replayed as well; the first call always runs eagerly, and a weight or
+buffer that it finds changed bumps the generation and so ends the replays.  The reference has no counterpart (it runs eager PyTorch, with host synchronisations
 in every quantiser call, qdiff/quant_layer.py:197-213).
 
 The tensor returned by a replayed call is a static buffer that the next call overwrites.
@@ -43,11 +45,14 @@ class GraphedModel:
             self._epoch = epoch
             self._calls = 0
         self._calls += 1
-        if self._calls <= EAGER_STEPS or _lib.TIMER is not None:
+        if self._calls == 1 or _lib.TIMER is not None:
             return qnn(x, t, context)
         _lib.require_cuda(x, "model input")
         key = (tuple(x.shape), None if context is None else tuple(context.shape), str(x.device))
         entry = self._graphs.get(key)
+        if self._calls <= EAGER_STEPS and (entry is None or
+                                           entry["generation"] != _lib.GENERATION[0]):
+            return qnn(x, t, context)
         if entry is not None and entry["generation"] != _lib.GENERATION[0]:
             # some layer moved a buffer since the capture (another input shape in between, a
             # repacked weight, a flag set on one layer): the recorded addresses are stale
