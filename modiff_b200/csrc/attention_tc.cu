@@ -5,19 +5,27 @@
 // split-bf16 operands as in gemm_bf16_tc.cu (hi*hi + hi*lo + lo*hi, fp32 accumulation in tensor
 // memory).  Scores and probabilities never touch global memory.
 //
-// A CTA owns 128 queries of one image at a time and walks the keys in blocks of 256:
-//   phase 1  tcgen05.mma (M=128, N=256) accumulates the block's scores in tensor-memory columns
-//            [0, 256) from TMA-fed q / k plane tiles;
-//   phase 2  the epilogue warps take the block's row maximum, fold it into the running maximum
-//            (online softmax: the output accumulator is rescaled in tensor memory when the
-//            maximum grows), and write the UNNORMALISED probabilities exp(s - max), 128 keys at a
-//            time, as two bf16 planes straight into shared memory in the 128-byte-swizzled
+// A CTA owns 128 queries of one image at a time and walks the keys in blocks of 128:
+//   phase 1  tcgen05.mma (M=128, N=128) accumulates a block's scores in one of two score buffers
+//            (tensor-memory columns [0, 128) and [128, 256)) from TMA-fed q / k plane tiles; the
+//            scores of block b + 1 are multiplied while the softmax works on block b;
+//   phase 2  the epilogue warps hold the block's scores in registers, fold its row maximum into the
+//            running maximum (online softmax: the output accumulator is rescaled in tensor memory
+//            in the warps where a maximum grew), and write the UNNORMALISED probabilities
+//            exp(s - max) as two bf16 planes straight into shared memory in the 128-byte-swizzled
 //            K-major layout an MMA A operand needs;
 //   phase 3  tcgen05.mma (N=channels<=256) accumulates P v in columns [256, 512), A operand
 //            = those shared-memory planes, B operand = TMA-fed v plane tiles;
 //   phase 4  after the last key block the epilogue divides by the row sum and writes
 //            out[image][channel][query].
-// Phase 1 of the next tile overlaps phase 4 of this one.  Every mbarrier wait is bounded.
+// A stage of the operand ring holds both planes of both operands of a 64-element K chunk (phase 1:
+// q and k, phase 3: v), i.e. all three products of it, so nothing is copied twice; heads of up to 64
+// channels keep the two q tiles in shared memory for all key blocks, and four smaller stages.
+// Bound: the softmax's instruction issue and the tensor pipe about equally.  Measured with the plane
+// splits in front, key blocks of 256 with one score buffer -> this: 16 heads x 40 channels x 4096
+// tokens 530 -> 360 us, 40 x 24 x 1024 119 -> 90 us, 16 x 80 x 1024 60 -> 47 us, 128 x 40 x 4096 queries
+// x 77 keys 220 -> 205 us, 256 x 256 x 256 162 -> 161 us; error against 64 bits unchanged (6e-6 - 1.6e-5).
+// Every mbarrier wait is bounded.
 #include "common.cuh"
 #include "tc_common.cuh"
 
@@ -26,9 +34,9 @@ namespace {
 
 constexpr int kChunkBytes = 128;                 // 64 bf16 of K per tile row
 constexpr int kATile = 128 * kChunkBytes;        // 16 KB: 128 queries
-constexpr int kBTileMax = 256 * kChunkBytes;     // 32 KB: up to 256 keys / channels
-constexpr int kStage = kATile + kBTileMax;       // 48 KB
-constexpr int kStages = 3;
+constexpr int kMaxStages = 4;
+constexpr int kRingBytes = 8 * kATile;           // 128 KB: 2 stages of 64 KB or 4 of 32 KB
+constexpr int kQBytes = 2 * kATile;              // resident q planes of heads of up to 64 channels
 constexpr int kPBytes = 2 * 2 * kATile;          // two planes x two 64-key chunks (128 keys) x 16 KB
 constexpr int kEpiWarps = 8;
 constexpr int kThreads = 64 + 32 * kEpiWarps;
@@ -38,17 +46,15 @@ struct AttnParams {
   int tkp;                      // keys padded to a multiple of 64
   int crow;                     // channel rows of the v planes (multiple of 64, <= 256)
   int cch;                      // 64-element K chunks of phase 1: ceil(cp / 64)
-  int n_s;                      // score columns per key block: min(256, tkp)
-  int nsb;                      // key blocks: ceil(tkp / 256)
+  int n_s;                      // score columns per key block: min(128, tkp)
+  int nsb;                      // key blocks: ceil(tkp / 128)
+  int q_resident;               // one K chunk: q stays in shared memory for all key blocks
+  int stages, stage_bytes;
   int q_tiles;                  // ceil(t / 128)
   int total_tiles;
   float scale;
   float* out;                   // [batch][c][t]
 };
-
-// the three products of a split-bf16 multiplication, (a part, b part): hi*hi, hi*lo, lo*hi
-__device__ inline int prod_a(int pr) { return pr == 2 ? 1 : 0; }
-__device__ inline int prod_b(int pr) { return pr == 1 ? 1 : 0; }
 
 // two floats -> packed bf16 pair (round to nearest even), first argument in the low half
 __device__ inline uint32_t bf16_pair(float lo_half, float hi_half) {
@@ -56,20 +62,35 @@ __device__ inline uint32_t bf16_pair(float lo_half, float hi_half) {
   asm("cvt.rn.bf16x2.f32 %0, %1, %2;" : "=r"(r) : "f"(hi_half), "f"(lo_half));
   return r;
 }
-// exp(x) for x <= 0 through the hardware exp2 (relative error ~2^-22, far below the 2^-16 the
+// 2^x for x <= 0 through the hardware exp2 (relative error ~2^-22, far below the 2^-16 the
 // split probabilities keep)
-__device__ inline float exp_neg(float x) {
+__device__ inline float exp2_neg(float x) {
   float r;
-  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x * 1.4426950408889634f));
+  asm("ex2.approx.ftz.f32 %0, %1;" : "=f"(r) : "f"(x));
   return r;
+}
+
+// The twelve MMAs of one K chunk: hi*hi, hi*lo, lo*hi of two planes each, one elected lane.
+__device__ inline void issue_chunk(uint32_t d_tmem, uint32_t a_hi, uint32_t a_lo, uint32_t b_hi,
+                                   uint32_t b_lo, uint32_t idesc, bool fresh) {
+  const uint64_t ah = make_smem_desc(a_hi), al = make_smem_desc(a_lo);
+  const uint64_t bh = make_smem_desc(b_hi), bl = make_smem_desc(b_lo);
+#pragma unroll
+  for (int k = 0; k < 4; ++k)
+    tc_mma_bf16(d_tmem, ah + (uint64_t)(2 * k), bh + (uint64_t)(2 * k), idesc, (fresh && k == 0) ? 0u : 1u);
+#pragma unroll
+  for (int k = 0; k < 4; ++k) tc_mma_bf16(d_tmem, ah + (uint64_t)(2 * k), bl + (uint64_t)(2 * k), idesc, 1u);
+#pragma unroll
+  for (int k = 0; k < 4; ++k) tc_mma_bf16(d_tmem, al + (uint64_t)(2 * k), bh + (uint64_t)(2 * k), idesc, 1u);
 }
 
 __global__ void __launch_bounds__(kThreads, 1)
 attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_constant__ CUtensorMap map_k,
                     const __grid_constant__ CUtensorMap map_v, const AttnParams p) {
   extern __shared__ __align__(1024) uint8_t smem_raw[];
-  __shared__ __align__(8) uint64_t bar_full[kStages], bar_empty[kStages];
-  __shared__ __align__(8) uint64_t bar_s_full, bar_p_ready, bar_p_free, bar_o_full, bar_o_empty;
+  __shared__ __align__(8) uint64_t bar_full[kMaxStages], bar_empty[kMaxStages];
+  __shared__ __align__(8) uint64_t bar_s_full[2], bar_q_full, bar_q_empty;
+  __shared__ __align__(8) uint64_t bar_p_ready, bar_p_free, bar_o_full, bar_o_empty;
   __shared__ uint32_t tmem_base_sh;
   __shared__ int abort_sh;
   __shared__ float red_max[2][128], red_sum[2][128];
@@ -80,14 +101,18 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
   const uint32_t raw = smem_u32(smem_raw);
   const uint32_t p_smem = raw;                       // probability planes
   const uint32_t ring = raw + kPBytes;               // operand stages
+  const uint32_t q_smem = ring + kRingBytes;         // resident q planes
 
   if (threadIdx.x == 0) {
     abort_sh = 0;
-    for (int s = 0; s < kStages; ++s) {
+    for (int s = 0; s < kMaxStages; ++s) {
       mbar_init(smem_u32(&bar_full[s]), 1);
       mbar_init(smem_u32(&bar_empty[s]), 1);
     }
-    mbar_init(smem_u32(&bar_s_full), 1);
+    mbar_init(smem_u32(&bar_s_full[0]), 1);
+    mbar_init(smem_u32(&bar_s_full[1]), 1);
+    mbar_init(smem_u32(&bar_q_full), 1);
+    mbar_init(smem_u32(&bar_q_empty), 1);
     mbar_init(smem_u32(&bar_p_ready), kEpiWarps);
     mbar_init(smem_u32(&bar_p_free), 1);
     mbar_init(smem_u32(&bar_o_full), 1);
@@ -110,37 +135,52 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
 
   if (warp == 0) {
     // ------------------------------------------------------------ TMA producer
+    // Stages in the order the MMA warp consumes them: scores(0), then scores(b + 1), values(b) ...
     if (lane == 0) {
       int stage = 0;
-      uint32_t phase = 0;
+      uint32_t phase = 0, qphase = 0;
       bool ok = true;
+      auto scores = [&](int img, int qt, int sb) {
+        for (int ch = 0; ch < p.cch && ok; ++ch) {
+          ok = mbar_wait(smem_u32(&bar_empty[stage]), phase ^ 1u, abort_flag);
+          if (!ok) return;
+          const uint32_t full = smem_u32(&bar_full[stage]);
+          const uint32_t dst = ring + stage * p.stage_bytes;
+          const uint32_t k_dst = dst + (p.q_resident ? 0 : 2 * kATile);
+          mbar_arrive_expect_tx(full, 2 * k_tile_bytes + (p.q_resident ? 0u : 2u * kATile));
+          for (int part = 0; part < 2; ++part) {
+            if (!p.q_resident)
+              tma_load_3d(dst + part * kATile, &map_q, full, ch * 64, qt * 128, img * 2 + part);
+            // key rows beyond tkp are filled with zeros by the copy and masked in the softmax
+            tma_load_3d(k_dst + part * kATile, &map_k, full, ch * 64, sb * 128, img * 2 + part);
+          }
+          if (++stage == p.stages) { stage = 0; phase ^= 1u; }
+        }
+      };
       for (int tile = blockIdx.x; tile < p.total_tiles && ok; tile += gridDim.x) {
         const int img = tile / p.q_tiles, qt = tile % p.q_tiles;
+        if (p.q_resident) {
+          ok = mbar_wait(smem_u32(&bar_q_empty), qphase ^ 1u, abort_flag);
+          qphase ^= 1u;
+          if (!ok) break;
+          const uint32_t full = smem_u32(&bar_q_full);
+          mbar_arrive_expect_tx(full, 2u * kATile);
+          for (int part = 0; part < 2; ++part)
+            tma_load_3d(q_smem + part * kATile, &map_q, full, 0, qt * 128, img * 2 + part);
+        }
+        scores(img, qt, 0);
         for (int sb = 0; sb < p.nsb && ok; ++sb) {
-          for (int ch = 0; ch < p.cch && ok; ++ch) {
-            for (int pr = 0; pr < 3; ++pr) {
-              ok = mbar_wait(smem_u32(&bar_empty[stage]), phase ^ 1u, abort_flag);
-              if (!ok) break;
-              const uint32_t full = smem_u32(&bar_full[stage]);
-              const uint32_t dst = ring + stage * kStage;
-              mbar_arrive_expect_tx(full, (uint32_t)kATile + k_tile_bytes);
-              tma_load_3d(dst, &map_q, full, ch * 64, qt * 128, img * 2 + prod_a(pr));
-              // key rows beyond tkp are filled with zeros by the copy and masked in the softmax
-              tma_load_3d(dst + kATile, &map_k, full, ch * 64, sb * 256, img * 2 + prod_b(pr));
-              if (++stage == kStages) { stage = 0; phase ^= 1u; }
-            }
-          }
-          const int kch = min(4, (p.tkp - sb * 256) >> 6);
+          if (sb + 1 < p.nsb) scores(img, qt, sb + 1);
+          const int kch = min(2, (p.tkp - sb * 128) >> 6);
           for (int kc = 0; kc < kch && ok; ++kc) {
-            for (int pr = 0; pr < 3; ++pr) {
-              ok = mbar_wait(smem_u32(&bar_empty[stage]), phase ^ 1u, abort_flag);
-              if (!ok) break;
-              const uint32_t full = smem_u32(&bar_full[stage]);
-              mbar_arrive_expect_tx(full, v_tile_bytes);
-              tma_load_3d(ring + stage * kStage + kATile, &map_v, full, sb * 256 + kc * 64, 0,
-                          img * 2 + prod_b(pr));
-              if (++stage == kStages) { stage = 0; phase ^= 1u; }
-            }
+            ok = mbar_wait(smem_u32(&bar_empty[stage]), phase ^ 1u, abort_flag);
+            if (!ok) break;
+            const uint32_t full = smem_u32(&bar_full[stage]);
+            mbar_arrive_expect_tx(full, 2 * v_tile_bytes);
+            for (int part = 0; part < 2; ++part)
+              tma_load_3d(ring + stage * p.stage_bytes + part * v_tile_bytes, &map_v, full,
+                          sb * 128 + kc * 64, 0, img * 2 + part);
+            if (++stage == p.stages) { stage = 0; phase ^= 1u; }
           }
         }
       }
@@ -153,71 +193,67 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
       const uint32_t idesc_s = make_idesc_bf16(128, p.n_s);
       const uint32_t idesc_o = make_idesc_bf16(128, p.crow);
       int stage = 0;
-      uint32_t phase = 0, tphase = 0, pphase = 0;
+      uint32_t phase = 0, tphase = 0, pphase = 0, qphase = 0;
       bool ok = true;
+      // scores of key block sb into its buffer.  The softmax has finished reading that buffer's
+      // previous scores: its p_ready for them preceded the values product issued before this one
+      // (or, for the first two blocks of a tile, the previous tile's last ones).
+      auto scores = [&](int sb) {
+        for (int ch = 0; ch < p.cch; ++ch) {
+          ok = mbar_wait(smem_u32(&bar_full[stage]), phase, abort_flag);
+          if (!ok) return;
+          tc_fence_after();
+          const uint32_t src = ring + stage * p.stage_bytes;
+          const uint32_t a_src = p.q_resident ? q_smem : src;
+          const uint32_t b_src = p.q_resident ? src : src + 2 * kATile;
+          if (elect_one()) {
+            issue_chunk(tmem_base + (uint32_t)((sb & 1) * 128), a_src, a_src + kATile, b_src, b_src + kATile,
+                        idesc_s, ch == 0);
+            tc_commit(smem_u32(&bar_empty[stage]));
+            if (ch == p.cch - 1) {
+              tc_commit(smem_u32(&bar_s_full[sb & 1]));
+              if (p.q_resident && sb == p.nsb - 1) tc_commit(smem_u32(&bar_q_empty));
+            }
+          }
+          __syncwarp();
+          if (++stage == p.stages) { stage = 0; phase ^= 1u; }
+        }
+      };
       for (int tile = blockIdx.x; tile < p.total_tiles; tile += gridDim.x) {
-        uint32_t fresh_pv = 1u;
-        for (int sb = 0; sb < p.nsb; ++sb) {
-          // phase 1: scores of this key block.  The softmax has finished reading the previous
-          // block's scores (its last p_ready preceded the MMAs issued just before this point).
-          for (int it = 0; it < 3 * p.cch; ++it) {
+        bool fresh_pv = true;
+        if (p.q_resident) {
+          ok = mbar_wait(smem_u32(&bar_q_full), qphase, abort_flag);
+          qphase ^= 1u;
+          if (!ok) break;
+        }
+        scores(0);
+        for (int sb = 0; sb < p.nsb && ok; ++sb) {
+          if (sb + 1 < p.nsb) scores(sb + 1);
+          if (!ok) break;
+          // phase 3: the probability planes of this block sit in shared memory; the tile's first
+          // product also needs the previous tile's output drained
+          ok = mbar_wait(smem_u32(&bar_p_ready), pphase, abort_flag);
+          pphase ^= 1u;
+          if (ok && fresh_pv) ok = mbar_wait(smem_u32(&bar_o_empty), tphase ^ 1u, abort_flag);
+          if (!ok) break;
+          tc_fence_after();
+          const int kch = min(2, (p.tkp - sb * 128) >> 6);
+          for (int kc = 0; kc < kch; ++kc) {
             ok = mbar_wait(smem_u32(&bar_full[stage]), phase, abort_flag);
             if (!ok) break;
             tc_fence_after();
-            const uint32_t a_src = ring + stage * kStage;
-            const uint64_t adesc = make_smem_desc(a_src);
-            const uint64_t bdesc = make_smem_desc(a_src + kATile);
+            const uint32_t a_src = p_smem + (uint32_t)(kc * kATile);     // plane stride 2 tiles
+            const uint32_t b_src = ring + stage * p.stage_bytes;
             if (elect_one()) {
-#pragma unroll
-              for (int k = 0; k < 4; ++k)
-                tc_mma_bf16(tmem_base, adesc + (uint64_t)(2 * k), bdesc + (uint64_t)(2 * k), idesc_s,
-                            (it > 0 || k > 0) ? 1u : 0u);
+              issue_chunk(tmem_base + 256u, a_src, a_src + 2 * kATile, b_src, b_src + v_tile_bytes, idesc_o,
+                          fresh_pv);
               tc_commit(smem_u32(&bar_empty[stage]));
+              if (kc == kch - 1) tc_commit(smem_u32(&bar_p_free));
             }
             __syncwarp();
-            if (++stage == kStages) { stage = 0; phase ^= 1u; }
+            fresh_pv = false;
+            if (++stage == p.stages) { stage = 0; phase ^= 1u; }
           }
-          if (!ok) break;
-          if (elect_one()) tc_commit(smem_u32(&bar_s_full));
-          __syncwarp();
-          // phase 3, 128 keys at a time: the probability planes of one half sit in shared memory
-          // while the epilogue warps wait to write the next half; the tile's first product also
-          // needs the previous tile's output drained
-          const int kch = min(4, (p.tkp - sb * 256) >> 6);
-          const int halves = (kch + 1) >> 1;
-          for (int kh = 0; kh < halves; ++kh) {
-            ok = mbar_wait(smem_u32(&bar_p_ready), pphase, abort_flag);
-            pphase ^= 1u;
-            if (ok && fresh_pv) ok = mbar_wait(smem_u32(&bar_o_empty), tphase ^ 1u, abort_flag);
-            if (!ok) break;
-            tc_fence_after();
-            const int kc_end = min(kch, 2 * kh + 2);
-            for (int kc = 2 * kh; kc < kc_end; ++kc) {
-              for (int pr = 0; pr < 3; ++pr) {
-                ok = mbar_wait(smem_u32(&bar_full[stage]), phase, abort_flag);
-                if (!ok) break;
-                tc_fence_after();
-                const uint64_t adesc =
-                    make_smem_desc(p_smem + (uint32_t)((prod_a(pr) * 2 + (kc & 1)) * kATile));
-                const uint64_t bdesc = make_smem_desc(ring + stage * kStage + kATile);
-                if (elect_one()) {
-#pragma unroll
-                  for (int k = 0; k < 4; ++k)
-                    tc_mma_bf16(tmem_base + 256u, adesc + (uint64_t)(2 * k), bdesc + (uint64_t)(2 * k),
-                                idesc_o, (fresh_pv && k == 0) ? 0u : 1u);
-                  tc_commit(smem_u32(&bar_empty[stage]));
-                }
-                __syncwarp();
-                fresh_pv = 0u;
-                if (++stage == kStages) { stage = 0; phase ^= 1u; }
-              }
-              if (!ok) break;
-            }
-            if (!ok) break;
-            if (elect_one()) tc_commit(smem_u32(&bar_p_free));
-            __syncwarp();
-          }
-          if (!ok) break;
         }
         if (!ok) break;
         if (elect_one()) tc_commit(smem_u32(&bar_o_full));
@@ -235,72 +271,80 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
     const uint32_t t_lane = tmem_base + ((uint32_t)(quarter * 32) << 16);
     const int ccols = p.crow >> 1;           // channel columns of this warp (multiple of 32)
     uint8_t* p_ptr = smem_raw;
-    uint32_t tphase = 0, sphase = 0, fphase = 0;
+    uint32_t tphase = 0, sphases = 0, fphase = 0;     // bit i of sphases: score buffer i
+    // scores in units of log2: exp(scale * s) = 2^(s * scale2)
+    const float scale2 = p.scale * 1.4426950408889634f;
     bool ok = true;
     for (int tile = blockIdx.x; tile < p.total_tiles; tile += gridDim.x) {
       const int img = tile / p.q_tiles, qt = tile % p.q_tiles;
       const int q = qt * 128 + row;
       float m_run = -INFINITY;      // running row maximum (the same in both warps of a pair)
-      float l_part = 0.0f;          // running sum of this warp's columns, in units of exp(-m_run)
+      float l_part = 0.0f;          // running sum of this warp's columns, in units of 2^(-m_run)
       for (int sb = 0; sb < p.nsb && ok; ++sb) {
-        const int keys_sb = min(256, p.tkp - sb * 256);
-        const int halves = (keys_sb + 127) >> 7;
-        ok = mbar_wait(smem_u32(&bar_s_full), sphase, abort_flag);
-        sphase ^= 1u;
+        const int nk = min(128, p.tkp - sb * 128) >> 1;       // this warp's keys: 32 or 64
+        ok = mbar_wait(smem_u32(&bar_s_full[sb & 1]), (sphases >> (sb & 1)) & 1u, abort_flag);
+        sphases ^= 1u << (sb & 1);
         if (!ok) break;
         tc_fence_after();
-        // Keys are handled 128 at a time (kh); inside a half the two warps of a lane quarter
-        // take half of its keys each (32 or 64 columns).
-        // ---- row maximum of this key block, folded into the running maximum
+        // ---- this warp's scores -> registers; row maximum folded into the running maximum
+        float s[64];
         float mx = -INFINITY;
-        for (int kh = 0; kh < halves; ++kh) {
-          const int nk = min(128, keys_sb - 128 * kh) >> 1;
-          for (int c0 = 0; c0 < nk; c0 += 32) {
-            const int col0 = 128 * kh + half * nk + c0;
-            int a[32];
-            tc_ld32(t_lane + (uint32_t)col0, a);
-            tc_wait_ld();
 #pragma unroll
-            for (int j = 0; j < 32; ++j)
-              if (sb * 256 + col0 + j < p.tk) mx = fmaxf(mx, __int_as_float(a[j]) * p.scale);
+        for (int c0 = 0; c0 < 64; c0 += 32) {
+          if (c0 < nk) {
+            const int col0 = half * nk + c0;
+            int a[32];
+            tc_ld32(t_lane + (uint32_t)((sb & 1) * 128 + col0), a);
+            tc_wait_ld();
+            const int left = p.tk - (sb * 128 + col0);        // real keys from this column on
+            if (left >= 32) {
+#pragma unroll
+              for (int j = 0; j < 32; ++j) {
+                s[c0 + j] = __int_as_float(a[j]) * scale2;
+                mx = fmaxf(mx, s[c0 + j]);
+              }
+            } else {
+#pragma unroll
+              for (int j = 0; j < 32; ++j) {
+                s[c0 + j] = __int_as_float(a[j]) * scale2;
+                if (j < left) mx = fmaxf(mx, s[c0 + j]);
+              }
+            }
           }
         }
         red_max[half][row] = mx;
         asm volatile("bar.sync 1, 256;" ::: "memory");
         const float m_new = fmaxf(m_run, fmaxf(red_max[0][row], red_max[1][row]));
-        // exp(m_run - m_new): 0 for the first block (m_run = -inf), 1 while the maximum stands
-        const float alpha = exp_neg(m_run - m_new);
+        // 2^(m_run - m_new): 0 for the first block (m_run = -inf), 1 while the maximum stands
+        const float alpha = exp2_neg(m_run - m_new);
         l_part *= alpha;
         m_run = m_new;
         // ---- exp, row sum, probabilities -> shared memory (K-major rows of 128 bytes, the
         //      16-byte chunk index XORed with row % 8: the layout TMA writes with 128-byte swizzle)
-        for (int kh = 0; kh < halves && ok; ++kh) {
-          // the MMAs that read the previous contents of the planes (and accumulated into the
-          // output columns) have completed
-          ok = mbar_wait(smem_u32(&bar_p_free), fphase ^ 1u, abort_flag);
-          fphase ^= 1u;
-          if (!ok) break;
-          if (kh == 0 && sb > 0) {
-            // online softmax: bring the accumulated output to the new maximum
-            tc_fence_after();
-            for (int c0 = 0; c0 < ccols; c0 += 32) {
-              int a[32];
-              tc_ld32(t_lane + 256u + (uint32_t)(half * ccols + c0), a);
-              tc_wait_ld();
-#pragma unroll
-              for (int j = 0; j < 32; ++j) a[j] = __float_as_int(__int_as_float(a[j]) * alpha);
-              tc_st32(t_lane + 256u + (uint32_t)(half * ccols + c0), a);
-            }
-            tc_wait_st();
-          }
-          const int nk = min(128, keys_sb - 128 * kh) >> 1;
-          for (int c0 = 0; c0 < nk; c0 += 32) {
-            const int col0 = 128 * kh + half * nk + c0;       // multiple of 32
-            const int key0 = sb * 256 + col0;
+        // the MMAs that read the previous contents of the planes (and accumulated into the
+        // output columns) have completed
+        ok = mbar_wait(smem_u32(&bar_p_free), fphase ^ 1u, abort_flag);
+        fphase ^= 1u;
+        if (!ok) break;
+        if (sb > 0 && __any_sync(0xffffffffu, alpha != 1.0f)) {
+          // online softmax: bring the accumulated output to the new maximum
+          tc_fence_after();
+          for (int c0 = 0; c0 < ccols; c0 += 32) {
             int a[32];
-            tc_ld32(t_lane + (uint32_t)col0, a);
+            tc_ld32(t_lane + 256u + (uint32_t)(half * ccols + c0), a);
             tc_wait_ld();
-            const int kc = (col0 >> 6) & 1;                   // 64-key chunk inside the half
+#pragma unroll
+            for (int j = 0; j < 32; ++j) a[j] = __float_as_int(__int_as_float(a[j]) * alpha);
+            tc_st32(t_lane + 256u + (uint32_t)(half * ccols + c0), a);
+          }
+          tc_wait_st();
+        }
+#pragma unroll
+        for (int c0 = 0; c0 < 64; c0 += 32) {
+          if (c0 < nk) {
+            const int col0 = half * nk + c0;                  // multiple of 32
+            const int left = p.tk - (sb * 128 + col0);
+            const int kc = col0 >> 6;                         // 64-key chunk of the block
             const int chunk0 = (col0 & 63) >> 3;              // first 16-byte chunk of the row: 0 or 4
             uint8_t* hi_row = p_ptr + (size_t)(0 * 2 + kc) * kATile + (size_t)row * 128;
             uint8_t* lo_row = p_ptr + (size_t)(1 * 2 + kc) * kATile + (size_t)row * 128;
@@ -313,8 +357,8 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
 #pragma unroll
                 for (int u = 0; u < 2; ++u) {
                   const int j = g8 * 8 + e + u;
-                  const float sv = __int_as_float(a[j]) * p.scale;
-                  pv[u] = (key0 + j < p.tk) ? exp_neg(sv - m_run) : 0.0f;
+                  pv[u] = exp2_neg(s[c0 + j] - m_run);
+                  if (left < 32) pv[u] = j < left ? pv[u] : 0.0f;
                   l_part += pv[u];
                 }
                 const uint32_t h = bf16_pair(pv[0], pv[1]);
@@ -327,12 +371,12 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
               *reinterpret_cast<uint4*>(lo_row + chunk * 16) = make_uint4(lw[0], lw[1], lw[2], lw[3]);
             }
           }
-          // a half with 64 keys fills one chunk; the MMA of this half then reads one chunk only
-          tc_fence_before();
-          asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
-          asm volatile("bar.sync 1, 256;" ::: "memory");
-          if (lane == 0) mbar_arrive(smem_u32(&bar_p_ready));
         }
+        // a block of 64 keys fills one chunk; its MMAs then read one chunk only
+        tc_fence_before();
+        asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
+        asm volatile("bar.sync 1, 256;" ::: "memory");
+        if (lane == 0) mbar_arrive(smem_u32(&bar_p_ready));
       }
       if (!ok) break;
       red_sum[half][row] = l_part;
@@ -408,8 +452,11 @@ extern "C" int modiff_attention_tc(const uint16_t* q_planes, const uint16_t* k_p
   p.tkp = tkp;
   p.crow = crow;
   p.cch = ceil_div(cp, 64);
-  p.n_s = tkp < 256 ? tkp : 256;
-  p.nsb = ceil_div(tkp, 256);
+  p.n_s = tkp < 128 ? tkp : 128;
+  p.nsb = ceil_div(tkp, 128);
+  p.q_resident = p.cch == 1 && crow == 64;
+  p.stage_bytes = p.q_resident ? 2 * kATile : 4 * kATile;
+  p.stages = kRingBytes / p.stage_bytes;
   p.q_tiles = ceil_div(t, 128);
   p.total_tiles = batch * p.q_tiles;
   p.scale = scale;
@@ -437,7 +484,7 @@ extern "C" int modiff_attention_tc(const uint16_t* q_planes, const uint16_t* k_p
     MODIFF_CUDA(cudaGetDevice(&dev));
     MODIFF_CUDA(cudaDeviceGetAttribute(&sm_count, cudaDevAttrMultiProcessorCount, dev));
   }
-  const size_t smem = (size_t)kPBytes + (size_t)kStages * kStage;
+  const size_t smem = (size_t)kPBytes + kRingBytes + (p.q_resident ? kQBytes : 0);
   static SmemLimit smem_limit;
   MODIFF_CUDA(raise_smem_limit(attention_tc_kernel, smem, smem_limit));
   const int grid = p.total_tiles < sm_count ? p.total_tiles : sm_count;
