@@ -4,8 +4,8 @@
 
 The decoder is not quantised in the reference and is not part of the timed sampling loop; it is
 here so that the latent configurations end in images.  Every layer runs on this package's own
-kernels in plain fp32: GroupNorm + SiLU (`modiff_groupnorm_silu`), convolutions as unquantised
-`QuantModule`s (`modiff_conv_fp32`, IEEE fp32, no TF32), nearest upsampling, the mid-block
+kernels at fp32 precision: convolutions as unquantised `QuantModule`s with the GroupNorm + SiLU,
+nearest upsampling and residual sum around them (`QuantModule.conv_plain`), the mid-block
 attention through `ops.attention`.  Module names and creation order are the reference's, so
 `torch.manual_seed` reproduces its random initialisation and its checkpoints' `state_dict`
 keys (`decoder.*`, `post_quant_conv.*`) load unchanged.  CUDA tensors only.

@@ -85,10 +85,13 @@ __device__ inline TileCoord decode_tile(int tile, const TcParams& p) {
   return t;
 }
 
-// TMA_EPI: the cached-output tile travels by bulk tensor copies (global -> shared before the
-// epilogue, shared -> global after it), so the epilogue threads touch only tensor memory and
-// shared memory.  Used for full-size layers with per-tensor scales and no bias; the generic
-// variant reads and writes o_hat directly and covers everything else.
+// TMA_EPI: the cached-output tile arrives by bulk tensor copies (global -> shared, during the products).
+// NCHW layers store the new values straight from registers - a lane is a pixel - and release the ring
+// slot as soon as it has been read; sending them back through the slot with a bulk store cost another
+// 0.25 - 0.45 us a launch (256 -> 256, 1x1 at 8x8, one image 6.1 -> 5.8 us; 768 -> 768 at 2x2, five
+// images, unsplit 25.2 -> 23.1 us).  Token-major layers, whose lanes are rows, keep the bulk store.  Used for
+// full-size layers with per-tensor scales and no bias; the generic variant reads and writes o_hat
+// directly and covers everything else.
 //
 // KSPLIT (layers with fewer tiles than SMs, e.g. 768 channels at 2x2 or 4x4): a cluster of
 // `p.ksplit` CTAs shares ONE tile.  Each CTA accumulates a contiguous part of the K range
@@ -141,7 +144,7 @@ igemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
     }
     for (int b = 0; b < kOSlots; ++b) {
       mbar_init(smem_u32(&bar_o_full[b]), 1);
-      mbar_init(smem_u32(&bar_o_empty[b]), 1);
+      mbar_init(smem_u32(&bar_o_empty[b]), p.row_epi ? 1 : kEpiWarps);
       mbar_init(smem_u32(&bar_o_ready[b]), kEpiWarps);
     }
     asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
@@ -275,9 +278,9 @@ igemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
     }
   } else if (warp == kStoreWarp) {
     // ------------------------------------------------------------ cached-output store warp
-    // Writes each finished half tile back with one bulk tensor store and hands the ring slot
-    // to the producer as soon as the store has read shared memory.
-    if (TMA_EPI && lane == 0) {
+    // Token-major layers: writes each finished half tile back with bulk tensor stores and hands the
+    // ring slot to the producer as soon as the stores have read shared memory.
+    if (TMA_EPI && p.row_epi && lane == 0) {
       int oslot = 0;
       uint32_t ophase = 0;
       bool ok = true;
@@ -286,14 +289,9 @@ igemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
         for (int hh = 0; hh < 2; ++hh) {
           ok = mbar_wait(smem_u32(&bar_o_ready[oslot]), ophase, abort_flag);
           if (!ok) break;
-          if (p.row_epi) {
-            for (int b2 = 0; b2 < 2; ++b2)
-              tma_store_2d(&map_o, obuf + oslot * kOHalfBytes + b2 * (kOHalfBytes / 2),
-                           t.nt * 128 + hh * 64 + b2 * 32, t.tn * p.bn);
-          } else {
-            tma_store_3d(&map_o, obuf + oslot * kOHalfBytes, t.th * p.bh * p.d.wo,
-                         t.nt * 128 + hh * 64, t.tn * p.bn);
-          }
+          for (int b2 = 0; b2 < 2; ++b2)
+            tma_store_2d(&map_o, obuf + oslot * kOHalfBytes + b2 * (kOHalfBytes / 2),
+                         t.nt * 128 + hh * 64 + b2 * 32, t.tn * p.bn);
           asm volatile("cp.async.bulk.commit_group;" ::: "memory");
           asm volatile("cp.async.bulk.wait_group.read 0;" ::: "memory");
           mbar_arrive(smem_u32(&bar_o_empty[oslot]));
@@ -384,6 +382,10 @@ igemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
           } else {
 #pragma unroll
             for (int j = 0; j < 32; ++j) v[j] = p.accumulate ? orow[j * tile_px] : 0.0f;
+            // the slot has been read: new values go to memory straight from registers (a lane is a
+            // pixel, so a warp writes runs of consecutive pixels per channel)
+            __syncwarp();
+            if (lane == 0) mbar_arrive(smem_u32(&bar_o_empty[oslot]));
           }
 #pragma unroll
           for (int seg = 0; seg < NSEG; ++seg) {
@@ -403,16 +405,27 @@ igemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
             for (int j4 = 0; j4 < 8; ++j4)
               *reinterpret_cast<float4*>(rbox + ((j4 ^ (row & 7)) << 4)) =
                   make_float4(v[4 * j4], v[4 * j4 + 1], v[4 * j4 + 2], v[4 * j4 + 3]);
+            // make the tile visible to the bulk-copy engine, then tell the store warp
+            asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
           } else {
+            const int n = t.tn * p.bn + ni;
+            const int co0 = t.nt * 128 + colbase;
+            if (n < p.g.batch) {
+              float* obase = p.o_hat + ((size_t)n * p.g.cout + co0) * howo + t.th * p.bh * p.d.wo + pl;
+              if (co0 + 32 <= p.g.cout) {
 #pragma unroll
-            for (int j = 0; j < 32; ++j) orow[j * tile_px] = v[j];
+                for (int j = 0; j < 32; ++j) obase[(size_t)j * howo] = v[j];
+              } else {
+#pragma unroll
+                for (int j = 0; j < 32; ++j)
+                  if (co0 + j < p.g.cout) obase[(size_t)j * howo] = v[j];
+              }
+            }
           }
           if (hh == 1) tc_fence_before();
-          // make the tile visible to the bulk-copy engine, then tell the store warp
-          asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
           __syncwarp();
           if (lane == 0) {
-            mbar_arrive(smem_u32(&bar_o_ready[oslot]));
+            if (p.row_epi) mbar_arrive(smem_u32(&bar_o_ready[oslot]));
             if (hh == 1) mbar_arrive(smem_u32(&bar_tmem_empty[buf]));   // accumulators consumed
           }
           if (++oslot == kOSlots) { oslot = 0; ophase ^= 1u; }
@@ -658,21 +671,6 @@ int launch_igemm_tc(const int8_t* codes, const int8_t* wcodes, int with_sum_rows
     MODIFF_CUDA(cudaGetDevice(&dev));
     MODIFF_CUDA(cudaDeviceGetAttribute(&sm_count, cudaDevAttrMultiProcessorCount, dev));
   }
-  // Few tiles and a long K range: clusters of 2 / 4 / 8 CTAs share each tile's K iterations, as
-  // long as the grid still fits the SMs at once and every CTA keeps at least three iterations.
-  p.ksplit = 1;
-  {
-    const char* e = getenv("MODIFF_TC_KSPLIT");     // 1 switches the split off (tests compare)
-    const int allow = e ? atoi(e) : 8;
-    const int iters = d.taps * p.chunks[0];
-    if (p.nseg == 1)
-      while (p.ksplit * 2 <= allow && p.ksplit < 8 && p.total_tiles * p.ksplit * 2 <= sm_count &&
-             iters >= 6 * p.ksplit * 2)
-        p.ksplit *= 2;
-    // the cluster's barriers and the exchange of partial sums cost about what 20 K iterations do
-    if (iters * (p.ksplit - 1) < 20 * p.ksplit) p.ksplit = 1;
-  }
-
   // The bulk-copy epilogue needs full-width row tiles of at least 4 pixels per image, per-tensor
   // scales, no bias and no accumulator dump.
   const int tile_px = p.bh * p.bw;
@@ -683,6 +681,23 @@ int launch_igemm_tc(const int8_t* codes, const int8_t* wcodes, int with_sum_rows
   const bool tma_epi_u = row_epi_u ||
                          (!per_sample && !bias && !acc_out && tile_px >= 4 && p.bw == d.wo &&
                           (d.ho * d.wo) % 4 == 0 && (((uintptr_t)o_hat & 15) == 0));
+  // Few tiles and a long K range: clusters of 2 / 4 / 8 CTAs share each tile's K iterations, as
+  // long as the grid still fits the SMs at once and every CTA keeps at least three iterations.
+  p.ksplit = 1;
+  {
+    const char* e = getenv("MODIFF_TC_KSPLIT");     // 1 switches the split off (tests compare)
+    const int allow = e ? atoi(e) : 8;
+    const int iters = d.taps * p.chunks[0];
+    // (token-major layers keep the bulk-copy epilogue: 512 rows x 5120 -> 1280 takes 16.6 us whole and
+    // 28.8 us split, whose epilogue touches 4 bytes of a row at a time)
+    if (p.nseg == 1 && !row_epi_u)
+      while (p.ksplit * 2 <= allow && p.ksplit < 8 && p.total_tiles * p.ksplit * 2 <= sm_count &&
+             iters >= 6 * p.ksplit * 2)
+        p.ksplit *= 2;
+    // the cluster's barriers and the exchange of partial sums cost about what 20 K iterations do
+    if (iters * (p.ksplit - 1) < 20 * p.ksplit) p.ksplit = 1;
+  }
+
   // what the layer would take without the K split decides how the split epilogue rounds
   p.fused_round = (row_epi_u || (tma_epi_u && g->cout >= 128)) ? 1 : 0;
   const bool row_epi = row_epi_u && p.ksplit == 1;

@@ -144,13 +144,6 @@ __device__ inline void tma_load_3d(uint32_t dst, const CUtensorMap* map, uint32_
       "l"(map), "r"(bar), "r"(c0), "r"(c1), "r"(c2)
       : "memory");
 }
-__device__ inline void tma_store_3d(const CUtensorMap* map, uint32_t src, int c0, int c1, int c2) {
-  asm volatile("cp.async.bulk.tensor.3d.global.shared::cta.bulk_group [%0, {%2, %3, %4}], [%1];" ::"l"(
-                   map),
-               "r"(src), "r"(c0), "r"(c1), "r"(c2)
-               : "memory");
-}
-
 // One lane of a fully active warp (the same lane every time it is asked).  The tensor-core
 // roles run their loops with ALL lanes, so that addresses and descriptors are warp-uniform
 // values the compiler can keep in uniform registers, and only the issue itself is elected.
