@@ -1168,6 +1168,9 @@ class QuantModule(nn.Module):
         members = self._group_members
         if not members or self.fwd_func is not F.linear or g.split != 0:
             return False
+        # whatever happens below, an earlier launch serves nobody any more: without this a group
+        # that is refused at one batch size would leave its members marked by another's launch
+        self._group_step += 1
         layers = [self] + members
         if g.batch * g.cin * sum(m.weight.shape[0] for m in layers) > \
                 self._GROUP_MAX_MACS * len(layers):
@@ -1197,7 +1200,6 @@ class QuantModule(nn.Module):
         _lib.call('modiff_linear_group', buf.codes.data_ptr(), buf.x_scale.data_ptr(), rows, g.cin,
                   tab['items'].data_ptr(), tab['block_map'].data_ptr(), tab['n_blocks'],
                   _lib.stream_ptr(), nbytes=nbytes, tag=g.key())
-        self._group_step += 1
         for m in members:
             m._group_served = (id(self), self._group_step)
         return True
