@@ -84,8 +84,8 @@ def test_outputs_are_a_fresh_layers_at_every_size(cuda, cin, couts, sizes):
 def _small_transformer(device):
     import modiff_b200 as m
     torch.manual_seed(0)
-    net = m.UNetModel(image_size=8, in_channels=4, out_channels=4, model_channels=320,
-                      attention_resolutions=[1], num_res_blocks=1, channel_mult=[2], num_heads=8,
+    net = m.UNetModel(image_size=8, in_channels=4, out_channels=4, model_channels=640,
+                      attention_resolutions=[1], num_res_blocks=1, channel_mult=[1], num_heads=8,
                       use_spatial_transformer=True, transformer_depth=1, context_dim=CIN,
                       legacy=False).eval()
     m.rerandomize_zero_tensors(net, seed=1)
