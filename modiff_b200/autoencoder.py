@@ -16,6 +16,7 @@ import torch.nn as nn
 from . import ops
 from ._lib import ModiffError
 from .quant_layer import QuantModule
+from .sampler import raise_on_device_status
 
 
 def _normalize(channels):
@@ -183,7 +184,13 @@ class FirstStageDecoder(nn.Module):
     """The decoding half of `AutoencoderKL` (ldm/models/autoencoder.py:285-333): the 1x1
     `post_quant_conv` from `embed_dim` to `z_channels`, then `decoder`.  `decode(z)` takes the
     sampler's latents; callers divide by the model's `scale_factor` first, as
-    `decode_first_stage` does (ldm/models/diffusion/ddpm.py)."""
+    `decode_first_stage` does (ldm/models/diffusion/ddpm.py).
+
+    After the last layer `decode` reads the device status word (`check_status`, default on) and
+    raises when a kernel gave up on a bounded wait, as the samplers do; that read waits for the
+    image.  Callers that queue several decodes or time them on the device pass False and check
+    once afterwards.  A decode that is being captured into a CUDA graph cannot read the word: the
+    caller does, after a replay (`modiff_b200.device_status`)."""
 
     def __init__(self, ddconfig=None, embed_dim=4):
         super().__init__()
@@ -193,9 +200,12 @@ class FirstStageDecoder(nn.Module):
         self.embed_dim = embed_dim
 
     @torch.no_grad()
-    def decode(self, z):
+    def decode(self, z, check_status=True):
         if not (torch.is_tensor(z) and z.is_cuda and z.dtype == torch.float32):
             raise ModiffError("the decoder runs on CUDA float32 tensors only (no CPU fallback)")
-        return self.decoder(_run_conv(self.post_quant_conv, z.contiguous()))
+        y = self.decoder(_run_conv(self.post_quant_conv, z.contiguous()))
+        if check_status and not torch.cuda.is_current_stream_capturing():
+            raise_on_device_status("decoding")
+        return y
 
     forward = decode

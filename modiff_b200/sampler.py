@@ -71,16 +71,18 @@ def step_coefficients(alphas, i, j, eta=0.0):
     return tuple(float(v) for v in (s1, s2, s3, c1, c2))
 
 
-def raise_on_device_status():
-    """Reads (and clears) the library's sticky device status word - one 4-byte device-to-host
-    copy, which waits for the stream - and raises when a kernel reported a failure: bit 0 a
-    bounded wait that ran out (the kernel returned early, its outputs are incomplete), bit 2 an
-    asymmetric zero point that did not fit the int8 code planes."""
+def raise_on_device_status(what="sampling"):
+    """Waits for the current stream, reads (and clears) the library's sticky device status word -
+    one 4-byte device-to-host copy - and raises when a kernel reported a failure: bit 0 a bounded
+    wait that ran out (the kernel returned early, its outputs are incomplete), bit 2 an asymmetric
+    zero point that did not fit the int8 code planes."""
+    if torch.cuda.is_initialized():
+        torch.cuda.current_stream().synchronize()   # the copy itself waits for blocking streams only
     status = _lib.device_status(reset=True)
     if status:
         raise _lib.ModiffError(
-            f"device status {status:#x} after sampling: a kernel gave up on a bounded wait or an "
-            "activation zero point did not fit its code plane; the samples are not valid")
+            f"device status {status:#x} after {what}: a kernel gave up on a bounded wait or an "
+            "activation zero point did not fit its code plane; the results are not valid")
 
 
 @torch.no_grad()

@@ -64,3 +64,35 @@ def test_decode_matches_the_reference(cuda):
         fs.decoder.conv_out.bias.add_(1.0)
     y2 = fs.decode(cases.decoder_latents(c).to(cuda))
     assert float((y2 - y - 1.0).abs().max()) < 1e-5
+
+
+@pytest.mark.gpu
+def test_decode_raises_when_a_kernel_gave_up(cuda):
+    """A wait that ran out (1 ms, nothing satisfies it) while the latents were being decoded is an
+    error and not an image; the read clears it, and it can be left to the caller."""
+    import modiff_b200 as m
+    from modiff_b200 import _lib
+    torch.manual_seed(0)
+    cfg = dict(double_z=True, z_channels=4, resolution=16, in_channels=3, out_ch=3, ch=32, ch_mult=(1, 2),
+               num_res_blocks=1, attn_resolutions=[], dropout=0.0)
+    fs = m.FirstStageDecoder(cfg).to(cuda)
+    z = torch.randn(1, 4, 8, 8, device=cuda)
+    want = fs.decode(z)
+    stream = torch.cuda.Stream()
+    for s in (torch.cuda.current_stream(), stream):
+        with torch.cuda.stream(s):
+            _lib.call('modiff_wait_probe', 1_000_000, None, _lib.stream_ptr())
+            with pytest.raises(m.ModiffError):
+                fs.decode(z)
+            assert torch.equal(fs.decode(z), want)
+            _lib.call('modiff_wait_probe', 1_000_000, None, _lib.stream_ptr())
+            fs.decode(z, check_status=False)
+            torch.cuda.synchronize()
+            assert m.device_status() & 1
+    # a decode can still be captured
+    graph = torch.cuda.CUDAGraph()
+    with torch.cuda.graph(graph):
+        y = fs.decode(z)
+    graph.replay()
+    torch.cuda.synchronize()
+    assert torch.equal(y, want) and m.device_status() == 0
