@@ -400,7 +400,8 @@ int modiff_conv_fp32(const float* x, const float* w_kn, const float* bias, float
                      const modiff_conv_geom* g, void* stream);
 
 /* The same convolution (stride 1, no split; qdiff/quant_layer.py:309-311) at fp32 precision on the
- * tensor cores: each fp32 operand as three bf16 planes that sum to it exactly.
+ * tensor cores: each fp32 operand as three bf16 planes that sum to it (exactly from 2^-103 on),
+ * six of the nine products of two operands (what is left out is at most 2^-24 of a product).
  *   modiff_f32_split_weights  w fp32 [cout][cin][kh][kw] -> weight planes (modiff_f32_weights_bytes)
  *   modiff_f32_split          x fp32 NCHW -> activation planes (modiff_f32_planes_bytes); on the way
  *       GroupNorm (groups > 0: gamma, beta, eps and modiff_f32_norm_bytes of work), SiLU, and, with
