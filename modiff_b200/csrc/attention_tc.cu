@@ -25,7 +25,8 @@
 // splits in front, key blocks of 256 with one score buffer -> this: 16 heads x 40 channels x 4096
 // tokens 530 -> 360 us, 40 x 24 x 1024 119 -> 90 us, 16 x 80 x 1024 60 -> 47 us, 128 x 40 x 4096 queries
 // x 77 keys 220 -> 205 us, 256 x 256 x 256 162 -> 161 us; error against 64 bits unchanged (6e-6 - 1.6e-5).
-// Every mbarrier wait is bounded.
+// Every mbarrier wait is bounded, and a softmax warp that gave up walks its loop to the end, so that no
+// other warp is left at a named barrier.
 #include "common.cuh"
 #include "tc_common.cuh"
 
@@ -280,18 +281,17 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
       const int q = qt * 128 + row;
       float m_run = -INFINITY;      // running row maximum (the same in both warps of a pair)
       float l_part = 0.0f;          // running sum of this warp's columns, in units of 2^(-m_run)
-      for (int sb = 0; sb < p.nsb && ok; ++sb) {
+      for (int sb = 0; sb < p.nsb; ++sb) {
         const int nk = min(128, p.tkp - sb * 128) >> 1;       // this warp's keys: 32 or 64
-        ok = mbar_wait(smem_u32(&bar_s_full[sb & 1]), (sphases >> (sb & 1)) & 1u, abort_flag);
+        if (ok) ok = mbar_wait_warp(smem_u32(&bar_s_full[sb & 1]), (sphases >> (sb & 1)) & 1u, abort_flag);
         sphases ^= 1u << (sb & 1);
-        if (!ok) break;
         tc_fence_after();
         // ---- this warp's scores -> registers; row maximum folded into the running maximum
         float s[64];
         float mx = -INFINITY;
 #pragma unroll
         for (int c0 = 0; c0 < 64; c0 += 32) {
-          if (c0 < nk) {
+          if (ok && c0 < nk) {
             const int col0 = half * nk + c0;
             int a[32];
             tc_ld32(t_lane + (uint32_t)((sb & 1) * 128 + col0), a);
@@ -323,10 +323,9 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
         //      16-byte chunk index XORed with row % 8: the layout TMA writes with 128-byte swizzle)
         // the MMAs that read the previous contents of the planes (and accumulated into the
         // output columns) have completed
-        ok = mbar_wait(smem_u32(&bar_p_free), fphase ^ 1u, abort_flag);
+        if (ok) ok = mbar_wait_warp(smem_u32(&bar_p_free), fphase ^ 1u, abort_flag);
         fphase ^= 1u;
-        if (!ok) break;
-        if (sb > 0 && __any_sync(0xffffffffu, alpha != 1.0f)) {
+        if (ok && sb > 0 && __any_sync(0xffffffffu, alpha != 1.0f)) {
           // online softmax: bring the accumulated output to the new maximum
           tc_fence_after();
           for (int c0 = 0; c0 < ccols; c0 += 32) {
@@ -341,7 +340,7 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
         }
 #pragma unroll
         for (int c0 = 0; c0 < 64; c0 += 32) {
-          if (c0 < nk) {
+          if (ok && c0 < nk) {
             const int col0 = half * nk + c0;                  // multiple of 32
             const int left = p.tk - (sb * 128 + col0);
             const int kc = col0 >> 6;                         // 64-key chunk of the block
@@ -376,15 +375,14 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
         tc_fence_before();
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         asm volatile("bar.sync 1, 256;" ::: "memory");
-        if (lane == 0) mbar_arrive(smem_u32(&bar_p_ready));
+        if (ok && lane == 0) mbar_arrive(smem_u32(&bar_p_ready));
       }
-      if (!ok) break;
       red_sum[half][row] = l_part;
       asm volatile("bar.sync 1, 256;" ::: "memory");
       const float inv = 1.0f / (red_sum[0][row] + red_sum[1][row]);
       // ---- output
-      ok = mbar_wait(smem_u32(&bar_o_full), tphase, abort_flag);
-      if (!ok) break;
+      if (ok) ok = mbar_wait_warp(smem_u32(&bar_o_full), tphase, abort_flag);
+      if (!ok) continue;               // on to the next tile's barriers
       tc_fence_after();
       for (int c0 = 0; c0 < ccols; c0 += 32) {
         int a[32];

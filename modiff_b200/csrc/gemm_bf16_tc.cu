@@ -218,7 +218,7 @@ gemm_bf16_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constan
         last_nt = t.nt;
       }
       if (ok) ok = mbar_wait(smem_u32(&bar_tmem_full[buf]), bphase, abort_flag);
-      if (!ok) break;
+      if (!ok) continue;               // on to the next tile's barriers
       tc_fence_after();
       const uint32_t t_row = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(buf * p.buf_cols);
       const int n = t.tn * p.bn + ni;

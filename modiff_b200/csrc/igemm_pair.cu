@@ -332,7 +332,8 @@ igemm_pair_kernel(const __grid_constant__ CUtensorMap map_a,
     int buf = 0, oslot = 0, last_nt = -1;
     uint32_t tphase = 0, ophase = 0;
     bool ok = true;
-    for (int tile = pair_id; tile < p.total_tiles; tile += num_pairs) {
+    int tile = pair_id;
+    for (; tile < p.total_tiles; tile += num_pairs) {
       const PairTile t = decode(tile, rank, p);
       if (t.nt != last_nt) {
         asm volatile("bar.sync 1, 256;" ::: "memory");
@@ -408,6 +409,14 @@ igemm_pair_kernel(const __grid_constant__ CUtensorMap map_a,
       }
       if (!ok) break;
       if (++buf == p.nbuf) { buf = 0; tphase ^= 1u; }
+    }
+    for (tile += num_pairs; tile < p.total_tiles; tile += num_pairs) {   // after a failed wait: as in igemm_halo.cu
+      const int nt = decode(tile, rank, p).nt;
+      if (nt != last_nt) {
+        asm volatile("bar.sync 1, 256;" ::: "memory");
+        asm volatile("bar.sync 1, 256;" ::: "memory");
+        last_nt = nt;
+      }
     }
   }
 

@@ -345,7 +345,7 @@ igemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
       }
 
       if (ok) ok = mbar_wait(smem_u32(&bar_tmem_full[buf]), bphase, abort_flag);
-      if (!ok) break;
+      if (!ok) continue;               // on to the next tile's barriers
       tc_fence_after();
       const uint32_t t_row = tmem_base + ((uint32_t)(quarter * 32) << 16) + (uint32_t)(buf * p.buf_cols);
       int rsum[2] = {0, 0};
@@ -430,7 +430,7 @@ igemm_tc_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant
           }
           if (++oslot == kOSlots) { oslot = 0; ophase ^= 1u; }
         }
-        if (!ok) break;
+        if (!ok) continue;
       } else if (KSPLIT) {
         // partial sums of this CTA's K range -> its own shared memory as [column][row] (the tile
         // ring is idle: every product that read it has completed); column 128 = the sum row
