@@ -161,6 +161,18 @@ inline cudaError_t raise_smem_limit(K kernel, size_t bytes, SmemLimit& st) {
 }
 #endif
 
+// SMs of the device the library first ran on (148 on a B200), for rules on how a grid fills it.
+inline int device_sms() {
+  static const int sms = [] {
+    int dev = 0, n = 0;
+    if (cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&n, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess)
+      return 148;
+    return n;
+  }();
+  return sms;
+}
+
 // Launch shape of the GroupNorm kernels for one (image, group) slab of `count` elements.  The
 // statistics are summed per thread and then over the block, so two kernels agree on the last
 // bit of mean and variance only when they use the same thread count.

@@ -124,6 +124,8 @@ groupnorm_silu_kernel(const float* __restrict__ x0, const float* __restrict__ x1
 // independent and issued four at a time) and the slices are added at the end.  (One block of 256
 // threads per image, each walking all channels of its pairs, took 46 us for one image of 16 tokens
 // and 256 channels.)
+// With images enough to fill the SMs by themselves the split costs more than it brings (every block
+// reads k and v again): attention_small_images_kernel.
 constexpr int kSmallQ = 8, kSmallThreads = 512;
 __global__ void __launch_bounds__(kSmallThreads)
 attention_small_kernel(const float* __restrict__ q, const float* __restrict__ k,
@@ -175,6 +177,40 @@ attention_small_kernel(const float* __restrict__ q, const float* __restrict__ k,
 #pragma unroll 4
     for (int j = 0; j < tk; ++j) r = fmaf(__ldg(vb + (size_t)ch * tk + j), sc[i][j], r);
     out[((size_t)b * c + ch) * t + i0 + i] = r;
+  }
+}
+
+// The same with one block per image, for many images: a thread walks the channels of its score pairs.
+__global__ void __launch_bounds__(256)
+attention_small_images_kernel(const float* __restrict__ q, const float* __restrict__ k,
+                              const float* __restrict__ v, float* __restrict__ out, int c, int t, int tk,
+                              float scale) {
+  __shared__ float sc[64][65];
+  const int b = blockIdx.x;
+  const float* qb = q + (size_t)b * c * t;
+  const float* kb = k + (size_t)b * c * tk;
+  const float* vb = v + (size_t)b * c * tk;
+  for (int e = threadIdx.x; e < t * tk; e += blockDim.x) {
+    const int i = e / tk, j = e % tk;
+    float acc = 0.0f;
+    for (int ch = 0; ch < c; ++ch) acc = fmaf(__ldg(qb + (size_t)ch * t + i), __ldg(kb + (size_t)ch * tk + j), acc);
+    sc[i][j] = acc * scale;
+  }
+  __syncthreads();
+  for (int i = threadIdx.x; i < t; i += blockDim.x) {
+    float mx = -INFINITY;
+    for (int j = 0; j < tk; ++j) mx = fmaxf(mx, sc[i][j]);
+    float sum = 0.0f;
+    for (int j = 0; j < tk; ++j) { const float e = expf(sc[i][j] - mx); sc[i][j] = e; sum += e; }
+    const float inv = 1.0f / sum;
+    for (int j = 0; j < tk; ++j) sc[i][j] *= inv;
+  }
+  __syncthreads();
+  for (int e = threadIdx.x; e < c * t; e += blockDim.x) {
+    const int ch = e / t, i = e % t;
+    float acc = 0.0f;
+    for (int j = 0; j < tk; ++j) acc = fmaf(__ldg(vb + (size_t)ch * tk + j), sc[i][j], acc);
+    out[(size_t)b * c * t + e] = acc;
   }
 }
 
@@ -426,6 +462,15 @@ int modiff_attention_small(const float* q, const float* k, const float* v, float
                            int c, int t, int tk, float scale, void* stream) {
   MODIFF_CHECK_ARG(q && k && v && out && batch > 0 && c > 0, "bad argument");
   MODIFF_CHECK_ARG(t > 0 && tk > 0 && t <= 64 && tk <= 64, "token counts %d x %d exceed 64", t, tk);
+  // Split / one block per image, us (images*heads x channels x queries x keys): 512 x 48 x 64 x 64
+  // 115 / 127, 768 168 / 168, 2048 547 / 374; 512 x 96 x 16 x 16 20 / 22, 768 29 / 25, 2048 68 / 52;
+  // 640 x 160 x 64 x 64 566 / 561.  Few pairs stay with the split (2048 x 96 x 4 x 4 14 / 24), and so
+  // do wide heads, whose operands no longer fit the L1 (640 x 512 x 64 x 64 2401 / 3775).
+  if (batch >= 4 * device_sms() && (t > kSmallQ || t * tk > 64) && c <= 256) {
+    attention_small_images_kernel<<<batch, 256, 0, (cudaStream_t)stream>>>(q, k, v, out, c, t, tk, scale);
+    MODIFF_LAUNCH_CHECK("attention_small_images_kernel");
+    return MODIFF_OK;
+  }
   int lg = 0;
   while ((1 << lg) < (t < kSmallQ ? t : kSmallQ) * tk) ++lg;
   attention_small_kernel<<<dim3(batch, ceil_div(t, kSmallQ)), kSmallThreads, 0, (cudaStream_t)stream>>>(

@@ -38,8 +38,10 @@ def test_grouped_linears_match_the_integer_sums(cuda, rows, cin, couts):
         assert torch.allclose(t[3].cpu(), want, rtol=2.0 ** -22, atol=2.0 ** -20)
 
 
+# images from four a SM on (592): one block each, except few pairs and wide heads
 @pytest.mark.parametrize("b,c,t,tk", [(1, 256, 16, 16), (3, 24, 64, 64), (2, 130, 7, 33), (5, 768, 4, 4),
-                                      (2, 64, 9, 1), (1, 64, 1, 64)])
+                                      (2, 64, 9, 1), (1, 64, 1, 64), (591, 24, 64, 64), (592, 24, 64, 64),
+                                      (600, 130, 7, 33), (600, 64, 9, 1), (600, 96, 4, 4), (600, 260, 9, 16)])
 def test_small_attention(cuda, b, c, t, tk):
     from modiff_b200 import _lib
     g = torch.Generator().manual_seed(t)
