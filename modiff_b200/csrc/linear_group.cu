@@ -9,8 +9,8 @@
 // channels is what bounds it, so the threads that the rows leave over share a row: KS lanes take
 // every KS-th 16-byte piece of it (and, with one or two rows, four warps take four channels
 // each), and their integer sums are added by shuffles.  Measured, one row per thread -> shared
-// rows: 2 rows, cin 1280, 22 layers 40.7 -> 13.7 us; 8 rows, cin 512 11.8 -> 6.7 us; 154 rows, cin 768,
-// 2 x 320 channels 21.8 -> 9.3 us; 256 rows unchanged (48 us).
+// rows: 2 rows, cin 1280, 22 layers 40.7 -> 13.7 us; 8 rows, cin 512 11.7 -> 6.1 us; 154 rows, cin 768,
+// 2 x 320 channels 21.8 -> 9.3 us; 256 rows, cin 512 49 -> 41 us.
 //
 // Arithmetic per layer: out = o_hat + (sum codes * (q - zp)) * delta_x * delta_w[c]
 // (qdiff/quant_layer.py:345-365), integer part exact.
@@ -23,9 +23,10 @@ constexpr int kGroupChannels = 16;
 constexpr int kGroupThreads = 256;
 
 // A thread owns CPT of the block's channels for one row and every 2^lg_ks-th piece of it; the
-// lanes of a row are neighbours.
+// lanes of a row are neighbours.  Four blocks a SM: with the 70 registers that the compiler takes
+// otherwise only three fit, and a grid of 445 - 592 blocks runs twice (64 rows, 3 x 320: 7.8 -> 12.6 us).
 template <int CPT>
-__global__ void __launch_bounds__(kGroupThreads)
+__global__ void __launch_bounds__(kGroupThreads, CPT == kGroupChannels ? 4 : 0)
 linear_group_kernel(const int8_t* __restrict__ codes, const float* __restrict__ x_scale, int rows,
                     int cin, int kp, int lg_ks, const modiff_linear_item* __restrict__ items,
                     const int32_t* __restrict__ block_map) {
@@ -111,11 +112,22 @@ extern "C" int modiff_linear_group(const int8_t* codes, const float* x_scale, in
   const size_t smem = (size_t)kGroupChannels * kp;
   const int cpt = rows <= 2 ? 4 : kGroupChannels;
   const int slots = kGroupThreads * cpt / kGroupChannels;      // threads per channel group
-  // lanes per row: what the rows leave over in one block, and more (hence more blocks along the
-  // rows) while the grid would not fill the SMs twice
-  int lg_ks = 0;
-  while (lg_ks < 5 && ((rows << (lg_ks + 1)) <= slots ||
-                       (int64_t)n_blocks * ceil_div(rows, slots >> lg_ks) < 2 * 148))
+  // Lanes per row: two, and further doublings where the rows leave the lanes over in one block or the
+  // grid stays below 2.75 blocks a SM: each doubling adds blocks along the rows, every block loads its 16
+  // weight rows again, and four of them are resident.  A row is cut into at most 16 pieces (one row
+  // alone into 32).  us for 1, 2, 4 .. 32 lanes, (rows, input channels, layers):
+  //   8, 512, 22 of 128 / 256     11.9  9.5  7.3  6.2  6.1  6.7     (one thread a row, 56 registers: 11.7)
+  //   64, 320, 3 x 320            10.3  8.4  7.4  6.2  6.6  7.8     (10.1)
+  //   96, 1280, 3 x 1280          35.9 30.0 34.1 28.4 33.2 45.4     (35.4)
+  //   154, 768, 2 x 640           24.7 19.4 15.5 13.6 16.3 22.5     (23.5)
+  //   192, 1280, 22 of 320 - 1280 178  158  187  197  250  380      (180)
+  //   256, 512, 22 of 128 / 256   50.1 40.7 44.0 50.8 65.6 98.7     (49.0)
+  //   512, 320, 3 x 320           17.2 17.7 18.7 20.3 27.5 38.8     (16.9)
+  const int max_lg = rows == 1 ? 5 : 4;
+  const int64_t max_blocks = 11 * device_sms() / 4;
+  int lg_ks = 1;
+  while (lg_ks < max_lg && ((rows << (lg_ks + 1)) <= slots ||
+                            (int64_t)n_blocks * ceil_div(rows, slots >> (lg_ks + 1)) <= max_blocks))
     ++lg_ks;
   dim3 grid(n_blocks, ceil_div(rows, slots >> lg_ks));
   cudaStream_t s = (cudaStream_t)stream;
