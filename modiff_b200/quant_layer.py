@@ -1144,10 +1144,16 @@ class QuantModule(nn.Module):
     # ------------------------------------------------------------------ grouped small linears
     group_small_linears = os.environ.get("MODIFF_LINEAR_GROUP", "1") != "0"
     _GROUP_MAX_ROWS = 512
-    # Multiply-adds per layer up to which one dp4a launch beats a tensor-core launch per layer
-    # (about 8.7 us each).  Measured, group / separate: 64 rows x 1280 -> 3 x 1280 (105 M a layer)
-    # 21 / 34 us, 128 rows (210 M) 32 / 26 us, 512 rows (839 M) 125 / 26 us.
-    _GROUP_MAX_MACS = 150e6
+    # Multiply-adds a layer (mean over layers of any widths) up to which one dp4a launch beats a
+    # tensor-core launch per layer: the second figure below 128 rows, where a separate GEMM takes its
+    # generic epilogue (11 - 13 us a layer against 7 - 9), and for more than 16 layers, which fill the
+    # SMs.  Measured, us group / separate: 128 rows x 1280 -> 3 x 1280 (210 M a layer) 33 / 25, 308 rows x
+    # 768 -> 2 x 640 (151 M) 23 / 15, 154 rows x 768 -> 12 x 1280 (151 M) 87 / 88, 160 (157 M) 89 / 88;
+    # 96 rows x 1280 -> 3 x 1280 (157 M) 30 / 39, -> 3 x 1600 (197 M) 38 / 39, -> 2560 + 1280 + 128
+    # (163 M) 30 / 40; 192 rows x 1280 -> 22 of 320 - 1280 (207 M) 158 / 190, 256 rows x 768 -> 25 of
+    # 384 - 1536 (196 M) 185 / 189, 308 rows (236 M) 225 / 188.  Between 85 M and 150 M two or three layers
+    # of 128 rows and more would be faster apart (256 rows x 768 -> 2 x 640, 126 M: 21 / 15).
+    _GROUP_MAX_MACS = (150e6, 200e6)
 
     def _group_register(self, member, g):
         """Called on the first step by a layer that shares this layer's codes.  Small linear
@@ -1172,8 +1178,8 @@ class QuantModule(nn.Module):
         # that is refused at one batch size would leave its members marked by another's launch
         self._group_step += 1
         layers = [self] + members
-        if g.batch * g.cin * sum(m.weight.shape[0] for m in layers) > \
-                self._GROUP_MAX_MACS * len(layers):
+        limit = self._GROUP_MAX_MACS[g.batch < 128 or len(layers) > 16]
+        if g.batch * g.cin * sum(m.weight.shape[0] for m in layers) > limit * len(layers):
             return False                     # each layer on the tensor cores
         for m in members:
             if m.a_hat is not self.a_hat or m.o_hat is None or m._wpack is None:

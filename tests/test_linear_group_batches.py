@@ -63,7 +63,8 @@ def test_every_output_is_written_once_an_evaluation(monkeypatch):
 
 @pytest.mark.gpu
 @pytest.mark.parametrize("cin,couts,sizes", [(CIN, (COUT, COUT), ROWS),
-                                             (1280, (1280, 1280, 1280), [64, 128, 64, 128])])
+                                             (1280, (1280, 1280, 1280), [64, 128, 96, 128]),
+                                             (1280, (320, 1280) * 9, [150, 200, 150])])
 def test_outputs_are_a_fresh_layers_at_every_size(cuda, cin, couts, sizes):
     import modiff_b200 as m
     used = _layers(cuda, cin, couts)
