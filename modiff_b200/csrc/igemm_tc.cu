@@ -688,8 +688,10 @@ int launch_igemm_tc(const int8_t* codes, const int8_t* wcodes, int with_sum_rows
     const char* e = getenv("MODIFF_TC_KSPLIT");     // 1 switches the split off (tests compare)
     const int allow = e ? atoi(e) : 8;
     const int iters = d.taps * p.chunks[0];
-    // (token-major layers keep the bulk-copy epilogue: 512 rows x 5120 -> 1280 takes 16.6 us whole and
-    // 28.8 us split, whose epilogue touches 4 bytes of a row at a time)
+    // (token-major layers keep the bulk-copy epilogue: a split one's touches 4 bytes of a row at a time.
+    // Where the rule below would split them, us whole / split: 5120 -> 1280 of 128 rows 16.4 / 19.4, 256
+    // rows 16.7 / 20.4, 308 rows 16.9 / 22.2, 512 rows 16.9 / 29.1; 4096 -> 4096 of 128 rows 14.7 / 20.5.  Below 128
+    // rows there is no such epilogue and the split stays: 64 rows, 5120 -> 1280 19.3 / 16.4.)
     if (p.nseg == 1 && !row_epi_u)
       while (p.ksplit * 2 <= allow && p.ksplit < 8 && p.total_tiles * p.ksplit * 2 <= sm_count &&
              iters >= 6 * p.ksplit * 2)
