@@ -535,14 +535,15 @@ attention_i8_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
     const bool magic_ok = p.c * 32768 < (1 << 22);
     uint32_t s_count = 0, p_count = 0, ophase = 0;
     bool ok = true;
-    for (int tile = blockIdx.x; tile < p.total_tiles; tile += gridDim.x) {
+    int tile = blockIdx.x, left = 0;                  // left: named barriers that a failed wait skipped
+    for (; tile < p.total_tiles; tile += gridDim.x) {
       const int img = tile / p.q_tiles, qt = tile % p.q_tiles;
       const int q = qt * 128 + row;
       // ---- pass A: exact integer row maximum
       int mx = INT_MIN;
       for (int j = 0; j < p.nkb && ok; ++j) {
         const uint32_t b = s_count & 1u, par = (s_count >> 1) & 1u;
-        ok = mbar_wait_warp(smem_u32(&bar_s_full[b]), par, abort_flag);
+        ok = mbar_wait(smem_u32(&bar_s_full[b]), par, abort_flag);
         if (!ok) break;
         tc_fence_after();
         {
@@ -564,6 +565,7 @@ attention_i8_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
         if (lane == 0) mbar_arrive(smem_u32(&bar_s_empty[b]));
         ++s_count;
       }
+      if (!ok) { left = 2; break; }
       red_max[part][row] = mx;
       asm volatile("bar.sync 1, %0;" ::"n"(32 * kEpiWarps) : "memory");
       int m_row = red_max[0][row];
@@ -574,9 +576,9 @@ attention_i8_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
       for (int j = 0; j < p.nkb && ok; ++j) {
         const uint32_t b = s_count & 1u, par = (s_count >> 1) & 1u;
         const uint32_t pb = p_count & 1u, ppar = (p_count >> 1) & 1u;
-        ok = mbar_wait_warp(smem_u32(&bar_s_full[b]), par, abort_flag);
+        ok = mbar_wait(smem_u32(&bar_s_full[b]), par, abort_flag);
         // the MMAs that read the previous contents of this weight tile have completed
-        if (ok) ok = mbar_wait_warp(smem_u32(&bar_p_free[pb]), ppar ^ 1u, abort_flag);
+        if (ok) ok = mbar_wait(smem_u32(&bar_p_free[pb]), ppar ^ 1u, abort_flag);
         if (!ok) break;
         tc_fence_after();
         uint8_t* prow = p_ptr + (size_t)pb * kTile + (size_t)row * kRowBytes;
@@ -605,6 +607,7 @@ attention_i8_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
         ++s_count;
         ++p_count;
       }
+      if (!ok) { left = 1; break; }
       red_sum[part][row] = l_part;
       asm volatile("bar.sync 1, %0;" ::"n"(32 * kEpiWarps) : "memory");
       int l_row = red_sum[0][row];
@@ -612,8 +615,8 @@ attention_i8_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
       for (int i = 1; i < kParts; ++i) l_row += red_sum[i][row];
       const float inv = __fdiv_rn(dv, (float)l_row);
       // ---- output
-      if (ok) ok = mbar_wait_warp(smem_u32(&bar_o_full), ophase, abort_flag);
-      if (!ok) continue;               // on to the next tile's barriers
+      ok = mbar_wait(smem_u32(&bar_o_full), ophase, abort_flag);
+      if (!ok) break;
       tc_fence_after();
       const int bimg = img / p.heads, head = img % p.heads;
       float* obase = p.out + (long long)bimg * p.ob + (long long)head * p.oh + (long long)q * p.ot;
@@ -639,6 +642,11 @@ attention_i8_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
       __syncwarp();
       if (lane == 0) mbar_arrive(smem_u32(&bar_o_empty));
       ophase ^= 1u;
+    }
+    // after a failed wait: the barriers of the remaining tiles and those skipped
+    for (tile += gridDim.x; tile < p.total_tiles; tile += gridDim.x) left += 2;
+    for (; left > 0; --left) {
+      asm volatile("bar.sync 1, %0;" ::"n"(32 * kEpiWarps) : "memory");
     }
   }
 

@@ -25,8 +25,8 @@
 // splits in front, key blocks of 256 with one score buffer -> this: 16 heads x 40 channels x 4096
 // tokens 530 -> 360 us, 40 x 24 x 1024 119 -> 90 us, 16 x 80 x 1024 60 -> 47 us, 128 x 40 x 4096 queries
 // x 77 keys 220 -> 205 us, 256 x 256 x 256 162 -> 161 us; error against 64 bits unchanged (6e-6 - 1.6e-5).
-// Every mbarrier wait is bounded, and a softmax warp that gave up walks its loop to the end, so that no
-// other warp is left at a named barrier.
+// Every mbarrier wait is bounded, and a softmax warp that gave up joins the rest of the named barriers, so
+// that no other warp is left at one.
 #include "common.cuh"
 #include "tc_common.cuh"
 
@@ -276,22 +276,24 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
     // scores in units of log2: exp(scale * s) = 2^(s * scale2)
     const float scale2 = p.scale * 1.4426950408889634f;
     bool ok = true;
-    for (int tile = blockIdx.x; tile < p.total_tiles; tile += gridDim.x) {
+    int tile = blockIdx.x, left = 0;                  // left: named barriers that a failed wait skipped
+    for (; tile < p.total_tiles; tile += gridDim.x) {
       const int img = tile / p.q_tiles, qt = tile % p.q_tiles;
       const int q = qt * 128 + row;
       float m_run = -INFINITY;      // running row maximum (the same in both warps of a pair)
       float l_part = 0.0f;          // running sum of this warp's columns, in units of 2^(-m_run)
       for (int sb = 0; sb < p.nsb; ++sb) {
         const int nk = min(128, p.tkp - sb * 128) >> 1;       // this warp's keys: 32 or 64
-        if (ok) ok = mbar_wait_warp(smem_u32(&bar_s_full[sb & 1]), (sphases >> (sb & 1)) & 1u, abort_flag);
+        ok = mbar_wait(smem_u32(&bar_s_full[sb & 1]), (sphases >> (sb & 1)) & 1u, abort_flag);
         sphases ^= 1u << (sb & 1);
+        if (!ok) { left = 2 * (p.nsb - sb) + 1; break; }
         tc_fence_after();
         // ---- this warp's scores -> registers; row maximum folded into the running maximum
         float s[64];
         float mx = -INFINITY;
 #pragma unroll
         for (int c0 = 0; c0 < 64; c0 += 32) {
-          if (ok && c0 < nk) {
+          if (c0 < nk) {
             const int col0 = half * nk + c0;
             int a[32];
             tc_ld32(t_lane + (uint32_t)((sb & 1) * 128 + col0), a);
@@ -323,9 +325,10 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
         //      16-byte chunk index XORed with row % 8: the layout TMA writes with 128-byte swizzle)
         // the MMAs that read the previous contents of the planes (and accumulated into the
         // output columns) have completed
-        if (ok) ok = mbar_wait_warp(smem_u32(&bar_p_free), fphase ^ 1u, abort_flag);
+        ok = mbar_wait(smem_u32(&bar_p_free), fphase ^ 1u, abort_flag);
         fphase ^= 1u;
-        if (ok && sb > 0 && __any_sync(0xffffffffu, alpha != 1.0f)) {
+        if (!ok) { left = 2 * (p.nsb - sb); break; }
+        if (sb > 0 && __any_sync(0xffffffffu, alpha != 1.0f)) {
           // online softmax: bring the accumulated output to the new maximum
           tc_fence_after();
           for (int c0 = 0; c0 < ccols; c0 += 32) {
@@ -340,7 +343,7 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
         }
 #pragma unroll
         for (int c0 = 0; c0 < 64; c0 += 32) {
-          if (ok && c0 < nk) {
+          if (c0 < nk) {
             const int col0 = half * nk + c0;                  // multiple of 32
             const int left = p.tk - (sb * 128 + col0);
             const int kc = col0 >> 6;                         // 64-key chunk of the block
@@ -375,14 +378,15 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
         tc_fence_before();
         asm volatile("fence.proxy.async.shared::cta;" ::: "memory");
         asm volatile("bar.sync 1, 256;" ::: "memory");
-        if (ok && lane == 0) mbar_arrive(smem_u32(&bar_p_ready));
+        if (lane == 0) mbar_arrive(smem_u32(&bar_p_ready));
       }
+      if (!ok) break;
       red_sum[half][row] = l_part;
       asm volatile("bar.sync 1, 256;" ::: "memory");
       const float inv = 1.0f / (red_sum[0][row] + red_sum[1][row]);
       // ---- output
-      if (ok) ok = mbar_wait_warp(smem_u32(&bar_o_full), tphase, abort_flag);
-      if (!ok) continue;               // on to the next tile's barriers
+      ok = mbar_wait(smem_u32(&bar_o_full), tphase, abort_flag);
+      if (!ok) break;
       tc_fence_after();
       for (int c0 = 0; c0 < ccols; c0 += 32) {
         int a[32];
@@ -399,6 +403,11 @@ attention_tc_kernel(const __grid_constant__ CUtensorMap map_q, const __grid_cons
       __syncwarp();
       if (lane == 0) mbar_arrive(smem_u32(&bar_o_empty));
       tphase ^= 1u;
+    }
+    // after a failed wait: the barriers of the remaining tiles and those skipped
+    for (tile += gridDim.x; tile < p.total_tiles; tile += gridDim.x) left += 2 * p.nsb + 1;
+    for (; left > 0; --left) {
+      asm volatile("bar.sync 1, 256;" ::: "memory");
     }
   }
 

@@ -66,13 +66,9 @@ __device__ inline bool mbar_wait(uint32_t bar, uint32_t parity, volatile int* ab
   return mbar_wait_limit(bar, parity, abort_flag, 2000000000ull);
 }
 // Warps that meet at a named barrier do not leave their loop after a failed wait without the rest of
-// its barriers: they walk it (or a loop of the barriers alone behind it) to the end, without waiting
-// or touching anything, whichever of them saw the failure first.  A warp that just left would keep
-// the others at its next barrier for ever.  The softmax warps wait with the following, which gives all
-// lanes one outcome: their key blocks branch on it around warp-wide instructions.
-__device__ inline bool mbar_wait_warp(uint32_t bar, uint32_t parity, volatile int* abort_flag) {
-  return __all_sync(0xffffffffu, mbar_wait(bar, parity, abort_flag));
-}
+// its barriers: they walk it to the end without waiting or touching anything, or join the remaining
+// barriers in a loop of their own behind it, whichever of them saw the failure first.  A warp that just
+// left would keep the others at its next barrier for ever.
 
 // ---------------------------------------------------------------- thread-block clusters
 __device__ inline uint32_t cluster_ctarank() {

@@ -1,6 +1,6 @@
 """Warps that meet at a named barrier must all reach it, also after one of them has given up on a
 bounded wait: in the kernels' sources no loop that holds such a barrier is left early, unless a loop
-with the same barriers, walked to its end, follows it."""
+of the remaining barriers, walked to its end, follows it."""
 import glob
 import os
 import re
@@ -33,9 +33,20 @@ def early_exits(text):
             k += 1
         loops.append((j, k, header))
     found = []
-    count = lambda b, e: len(BARRIER.findall(text[b:e]))
-    followed = lambda end, n: any(text[end:b].count('{') == 0 and text[end:b].count('}') == 0 and
-                                  b > end and count(b, e) == n for b, e, _ in loops)
+
+    def same_scope(a, b):                 # text from a to b closes no scope that is open at a
+        depth = 0
+        for ch in text[a:b]:
+            depth += {'{': 1, '}': -1}.get(ch, 0)
+            if depth < 0:
+                return False
+        return True
+
+    def followed(beg, end):               # by a loop with barriers, behind this loop or one around it
+        around = [e for b, e, _ in loops if b <= beg and end <= e]
+        return any(same_scope(a, b) and BARRIER.search(text[b:e]) and not re.search(r'\b(break|return)\b', text[b:e])
+                   for a in around for b, e, _ in loops if b > a)
+
     line = lambda pos: text.count('\n', 0, pos) + 1
     for beg, end, header in loops:
         body = text[beg:end]
@@ -48,7 +59,7 @@ def early_exits(text):
             inner = [(b, e) for b, e, _ in loops if beg < b < pos < e]
             # a break of an inner loop without a barrier leaves only that loop (loop bodies without
             # braces hold one statement, in which no kernel breaks)
-            if m.group(1) == 'break' and (inner or followed(end, count(beg, end))):
+            if m.group(1) == 'break' and (inner or followed(beg, end)):
                 continue
             found.append((line(pos), m.group(1)))
     return found
