@@ -166,3 +166,39 @@ def test_a_lost_plane_or_product_would_be_seen(b, cin, cout, hw, k, positive):
     assert error([(0, 0), (0, 1), (1, 0), (1, 1)]) > 1.5 * err_chain          # two planes
     for lost in six[1:]:
         assert error([p for p in six if p != lost]) > 1.5 * err_chain, lost
+
+
+@pytest.mark.gpu
+@pytest.mark.parametrize("form", ["conv1d_k1_pow2", "conv1d_k1", "conv1d_k3", "implicit_pad", "channels_last", "sliced",
+                                  "offset", "weights_channels_last", "no_bias"])
+def test_every_form_of_the_layer_agrees_with_the_fp32_kernel(cuda, form):
+    """Orders, strides, alignments and paddings that the unquantised layer takes, against modiff_conv_fp32
+    on the same layer: both are fp32 sums of 32 - 288 products, 1e-5 of the largest output apart at most
+    (their own errors are below 1e-6 of the root mean square)."""
+    torch.manual_seed(11)
+    if form.startswith("conv1d"):
+        k = 3 if form.endswith("k3") else 1
+        conv = torch.nn.Conv1d(32, 24, k, padding=k // 2)
+        x = torch.randn(2, 32, 64 if form.endswith("pow2") else 21, device=cuda)
+    else:
+        conv = torch.nn.Conv2d(32, 24, 3, padding=0 if form == "implicit_pad" else 1, bias=form != "no_bias")
+        x = torch.randn(2, 32, 10, 7, device=cuda)
+    conv = conv.to(cuda)
+    if form == "weights_channels_last":
+        conv = conv.to(memory_format=torch.channels_last)
+    layer = _layer(conv)
+    if form == "implicit_pad":
+        layer.implicit_pad = (0, 1, 0, 1)          # right and bottom, as the UNet's downsampling pads
+    plain_in = x
+    if form == "channels_last":
+        x = x.contiguous(memory_format=torch.channels_last)
+    elif form == "sliced":
+        x = torch.cat([x, x], dim=1)[:, :32]
+    elif form == "offset":                         # contiguous, four bytes off a 16-byte boundary
+        x = torch.cat([x.new_zeros(1), x.flatten()])[1:].view(x.shape)
+        assert x.data_ptr() % 16 == 4
+    y = layer(x)
+    g = layer._geom(plain_in, 0)
+    ref = torch.empty_like(y)
+    layer._conv_fp32(plain_in, layer._org_weights_kn(), layer.org_bias, g, ref)
+    assert float((y - ref).abs().max()) <= 1e-5 * float(ref.abs().max())
